@@ -200,7 +200,7 @@ const float *dct_eigen(int M)
 enum BufId {
     B_PHASE, B_AMP, B_PHU, B_CHG, B_CUT, B_GOLD, B_U, B_F2, B_COUNTS, B_G, B_T1, B_S, B_BGF, B_DCT, B_MASK, B_GEOM,
     B_CARRIER, B_KEY, B_SCRATCH, B_HOLO, B_BG, B_RI, B_GSTATE, B_GLIST, B_GSTATUS, B_FASTW, B_FASTIN, B_TMP, B_GWORK,
-    B_TMASK, B_TCOUNT, B_TVALS, B_QMAG, B_FIT, B_PV, B_PG, B_PV2, B_PG2, B_PVP, B_PPART, B_PCTL, B_PHIST, B_STAGE, B_STAGEBG, B_TPRE, B_RI2, B_XPREV, NBUF
+    B_TMASK, B_TCOUNT, B_TVALS, B_QMAG, B_FIT, B_PV, B_PG, B_PV2, B_PG2, B_PVP, B_PPART, B_PCTL, B_PHIST, B_STAGE, B_STAGEBG, B_TPRE, B_RI2, B_XPREV, B_TACT, NBUF
 };
 
 // Stage boundaries recorded with CUDA events when timing is enabled.
@@ -680,14 +680,14 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
     la.mask = mask;
     la.out = ri;
     la.R = R;
-    la.inv_n3 = (float)(1.0 / ((double)R * R * R));
     la.k2 = (float)k2;
     la.n_med = (float)n_med;
     la.n_med2 = (float)(n_med * n_med);
-    la.s1 = (float)(-1.0 / ((double)R * R * R * k2));
+    la.inv_r = (float)(1.0 / R);
     la.s2 = (float)(-k2 / (n_med * n_med));
     la.err = c->d_err;
     CK(ensure_tuned(R, check_mode, s), "autotune loop passes");
+    // B_TACT: the caller made it and cleared its header
     // the z pass reads the measured samples packed per tile when its plan allows
     const int TB = loop_ztile(R);
     la.packed = 0;
@@ -698,13 +698,14 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
         CK(ensure(c, B_TPRE, sizeof(int) * tiles * R), "alloc packed prefixes");
         CK(ensure(c, B_TVALS, sizeof(float2) * r3), "alloc packed values");
         CK(pack_measured(F2, check_mode == CTDM_CHECK_MASK ? mask : nullptr, R, TB, B<uint32_t>(c, B_TMASK),
-                         B<int>(c, B_TCOUNT), B<int>(c, B_TPRE), B<float2>(c, B_TVALS), s),
+                         B<int>(c, B_TCOUNT), B<int>(c, B_TPRE), B<float2>(c, B_TVALS), R > 128 ? B<int>(c, B_TACT) : nullptr, s),
            "pack measured samples");
         la.tmask = B<uint32_t>(c, B_TMASK);
         la.tcount = B<int>(c, B_TCOUNT);
         la.tprefix = B<int>(c, B_TPRE);
         la.tvals = B<float2>(c, B_TVALS);
         la.packed = 1;
+        active_view(la, B<int>(c, B_TACT), R);
     }
     la.xprev = nullptr;
     la.beta = 0.f;
@@ -719,7 +720,11 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
         t_k = t_n;
     };
     StageTimer &tm = c->timer;
-    if (loop_scheme(R) >= 1) {
+    // G holds z lines normalised by 1 / R (g_scale of the mapping, the z passes); the y
+    // inverse line pass normalises too, the plane pass leaves 1 / R^2 to s1
+    const bool planes = loop_scheme(R) >= 1;
+    la.s1 = (float)(-1.0 / ((planes ? (double)R * R : (double)R) * k2));
+    if (planes) {
         // plane + z passes, 8- or 4-CTA clusters per plane (schemes 1, 2; the plane pass
         // records under the x-pass stage)
         for (int it = 0; it < iters; it++) {
@@ -733,7 +738,10 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
         tm.mark(S_XFINAL, s);
         return CTDM_OK;
     }
+    const int *xactive = la.xactive;
+    la.xactive = nullptr;   // F2 may hold values that the loop does not keep: every column
     CK(launch_ypass(la, true, s), "y inverse pass");
+    la.xactive = xactive;
     tm.mark(S_YINV, s);
     for (int it = 0; it < iters; it++) {
         next_beta();
@@ -847,6 +855,7 @@ static ctdm_status pipeline_core(ctdm_ctx *c, const ctdm_params *p, int A, int M
     CK(ensure(c, B_U, sizeof(float2) * A * rr), "alloc spectra");
     CK(ensure(c, B_F2, sizeof(float2) * r3), "alloc F2");
     CK(ensure(c, B_G, sizeof(float2) * r3), "alloc G");
+    CK(ensure(c, B_TACT, sizeof(int) * active_ints(R)), "alloc active tiles");
     const bool mask_mode = p->check_mode == CTDM_CHECK_MASK;
     CK(ensure(c, B_COUNTS, mask_mode ? sizeof(uint32_t) * r3 : 0), "alloc counts");
     CK(ensure(c, B_MASK, mask_mode ? r3 : 0), "alloc mask");
@@ -964,8 +973,10 @@ static ctdm_status pipeline_core(ctdm_ctx *c, const ctdm_params *p, int A, int M
     ea.dx = (float)p->dx;
     ea.F2 = B<float2>(c, B_F2);
     ea.G = B<float2>(c, B_G);
+    ea.g_scale = (float)(1.0 / R);
     ea.counts = mask_mode ? B<uint32_t>(c, B_COUNTS) : nullptr;
     ea.mask = mask_mode ? B<uint8_t>(c, B_MASK) : nullptr;
+    ea.active = B<int>(c, B_TACT);
     CK(launch_ewald(ea, s), "ewald mapping");
     tm.mark(S_EWALD, s);
     if (feed && feed->front_done) CK(cudaEventRecord(feed->front_done, s), "front end done");
@@ -1591,8 +1602,10 @@ extern "C" ctdm_status ctdm_positivity_ex(ctdm_ctx *c, int R, int iterations, in
     const long rr = (long)R * R, r3 = rr * R;
     CK(ensure(c, B_G, sizeof(float2) * r3), "alloc G");
     float2 *G = B<float2>(c, B_G);
-    CK(cudaMemcpyAsync(G, d_F2, sizeof(float2) * r3, cudaMemcpyDeviceToDevice, s), "copy F2");
-    CK(fft_cols(G, R, rr, (int)rr, 0, rr, true, s), "z inverse");
+    CK(fft_cols_from(reinterpret_cast<const float2 *>(d_F2), G, R, rr, (int)rr, 0, rr, true, (float)(1.0 / R), s),
+       "z inverse");
+    CK(ensure(c, B_TACT, sizeof(int) * active_ints(R)), "alloc active tiles");
+    CK(cudaMemsetAsync(c->buf[B_TACT], 0, sizeof(int) * active_head(R), s), "clear active tiles");
     const uint8_t *mask = nullptr;
     if (check_mode == CTDM_CHECK_MASK) {
         CK(ensure(c, B_MASK, r3), "alloc mask");

@@ -133,9 +133,10 @@ __global__ void __launch_bounds__(Plan<L>::THREADS) rows_kernel(float2 *data, co
     store_rows<L>(data, buf, line0, nlines);
 }
 
+// src may be data itself (in place); the result is scaled by `scale`.
 template <int L, bool INV>
-__global__ void __launch_bounds__(Plan<L>::THREADS) cols_kernel(float2 *data, const float2 *__restrict__ tw, long nlines,
-                                                                int nx, long plane, long ld)
+__global__ void __launch_bounds__(Plan<L>::THREADS) cols_kernel(const float2 *src, float2 *data, const float2 *__restrict__ tw,
+                                                                long nlines, int nx, long plane, long ld, float scale)
 {
     using P = Plan<L>;
     using En = fftl::Ends<L>;
@@ -148,11 +149,12 @@ __global__ void __launch_bounds__(Plan<L>::THREADS) cols_kernel(float2 *data, co
     float2 v[P::E];
 #pragma unroll
     for (int i = 0; i < P::E; i++)
-        v[i] = ok ? __ldcs(&data[base + (long)fftl::slot_pos<L, P::T, En::F>(i, t) * ld]) : make_float2(0.f, 0.f);
+        v[i] = ok ? __ldcs(&src[base + (long)fftl::slot_pos<L, P::T, En::F>(i, t) * ld]) : make_float2(0.f, 0.f);
     P::template seq<INV, false, false>(buf, v, tw);
     if (!ok) return;
 #pragma unroll
-    for (int i = 0; i < P::E; i++) __stcs(&data[base + (long)fftl::slot_pos<L, P::T, En::Rv>(i, t) * ld], v[i]);
+    for (int i = 0; i < P::E; i++)
+        __stcs(&data[base + (long)fftl::slot_pos<L, P::T, En::Rv>(i, t) * ld], cscale(v[i], scale));
 }
 
 // Large dynamic shared memory opt-in and the largest shared-memory carveout, so
@@ -183,7 +185,8 @@ static cudaError_t rows_launch(float2 *data, long nlines, bool inv, cudaStream_t
 }
 
 template <int L>
-static cudaError_t cols_launch(float2 *data, long nlines, int nx, long plane, long ld, bool inv, cudaStream_t s)
+static cudaError_t cols_launch(const float2 *src, float2 *data, long nlines, int nx, long plane, long ld, bool inv,
+                               float scale, cudaStream_t s)
 {
     using P = Plan<L>;
     const size_t smem = fftl::smem_bytes<L>();
@@ -191,7 +194,7 @@ static cudaError_t cols_launch(float2 *data, long nlines, int nx, long plane, lo
     auto k = inv ? cols_kernel<L, true> : cols_kernel<L, false>;
     cudaError_t e = prep_launch<L>(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<(unsigned)grid, P::THREADS, smem, s>>>(data, twiddles(L), nlines, nx, plane, ld); note_launch();
+    k<<<(unsigned)grid, P::THREADS, smem, s>>>(src, data, twiddles(L), nlines, nx, plane, ld, scale); note_launch();
     return cudaGetLastError();
 }
 
@@ -202,7 +205,13 @@ cudaError_t fft_rows(float2 *data, int L, long nlines, bool inverse, cudaStream_
 
 cudaError_t fft_cols(float2 *data, int L, long nlines, int nx, long plane, long ld, bool inverse, cudaStream_t s)
 {
-    CTDM_DISPATCH_L(L, cols_launch, data, nlines, nx, plane, ld, inverse, s)
+    return fft_cols_from(data, data, L, nlines, nx, plane, ld, inverse, 1.0f, s);
+}
+
+cudaError_t fft_cols_from(const float2 *src, float2 *dst, int L, long nlines, int nx, long plane, long ld,
+                          bool inverse, float scale, cudaStream_t s)
+{
+    CTDM_DISPATCH_L(L, cols_launch, src, dst, nlines, nx, plane, ld, inverse, scale, s)
 }
 
 __global__ void scale_kernel(float2 *d, long n, float s, bool conj)
@@ -296,6 +305,8 @@ __global__ void __launch_bounds__(Plan<L>::THREADS) ewald_kernel(EwaldArgs a, co
     const long line0 = (long)blockIdx.x * P::B;   // line = x + R*y, B consecutive x
     for (int e = threadIdx.x; e < P::B * P::LP; e += P::THREADS) buf[e] = make_float2(0.f, 0.f);
     for (int e = threadIdx.x; e < P::B * L; e += P::THREADS) cnt[e] = 0u;
+    if (a.active && blockIdx.x == 0)
+        for (int e = threadIdx.x; e < active_head(L); e += P::THREADS) a.active[e] = 0;
     for (int e = threadIdx.x; e < a.A; e += P::THREADS) {
         geo[e] = a.geom[e];
         if constexpr (FI) {
@@ -382,7 +393,7 @@ __global__ void __launch_bounds__(Plan<L>::THREADS) ewald_kernel(EwaldArgs a, co
         const int b = threadIdx.x % P::B, t = threadIdx.x / P::B;
         const long base = line0 + b;
 #pragma unroll
-        for (int i = 0; i < P::E; i++) a.G[base + (long)fftl::slot_pos<L, P::T, fftl::Ends<L>::Rv>(i, t) * rr] = v[i];
+        for (int i = 0; i < P::E; i++) a.G[base + (long)fftl::slot_pos<L, P::T, fftl::Ends<L>::Rv>(i, t) * rr] = cscale(v[i], a.g_scale);
     }
 }
 
@@ -407,7 +418,7 @@ static cudaError_t ewald_launch(const EwaldArgs &a, cudaStream_t s)
 template <int TB>
 __global__ void __launch_bounds__(256) pack_measured_kernel(const float2 *__restrict__ F2,
                                                            const uint8_t *__restrict__ mask, int R, uint32_t *tmask,
-                                                           int *tcount, int *tprefix, float2 *tvals)
+                                                           int *tcount, int *tprefix, float2 *tvals, int *active)
 {
     extern __shared__ int spre[];   // R prefixes, then 8 warp totals
     int *swarp = spre + R;
@@ -466,7 +477,14 @@ __global__ void __launch_bounds__(256) pack_measured_kernel(const float2 *__rest
         if (z < R) spre[z] = run;
         run += own[k];
     }
-    if (threadIdx.x == 255) tcount[tile] = run;
+    if (threadIdx.x == 255) {
+        tcount[tile] = run;
+        if (active && run > 0) {
+            // the list's order only decides which CTA takes which tile
+            active[active_head(R) + atomicAdd(&active[0], 1)] = (int)tile;
+            for (int x = 0; x < TB; x += 8) active[4 + (int)(line0 % R + x) / 8] = 1;
+        }
+    }
     __syncthreads();
     for (int z = threadIdx.x; z < R; z += 256) tprefix[tile * R + z] = spre[z];
     float2 *tv = tvals + tile * (long)TB * R;
@@ -481,15 +499,15 @@ __global__ void __launch_bounds__(256) pack_measured_kernel(const float2 *__rest
 }
 
 cudaError_t pack_measured(const float2 *F2, const uint8_t *mask, int R, int TB, uint32_t *tmask, int *tcount,
-                          int *tprefix, float2 *tvals, cudaStream_t s)
+                          int *tprefix, float2 *tvals, int *active, cudaStream_t s)
 {
     if (R > 768) return cudaErrorInvalidValue;
     const unsigned tiles = (unsigned)((long)R * R / TB);
     const size_t smem = sizeof(int) * (R + 8);
     switch (TB) {
-    case 8: pack_measured_kernel<8><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals); break;
-    case 16: pack_measured_kernel<16><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals); break;
-    case 32: pack_measured_kernel<32><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals); break;
+    case 8: pack_measured_kernel<8><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active); break;
+    case 16: pack_measured_kernel<16><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active); break;
+    case 32: pack_measured_kernel<32><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active); break;
     default: return cudaErrorInvalidValue;
     }
     note_launch();

@@ -35,9 +35,11 @@ struct EwaldArgs {
     float fm02s;            // (fm0/df)^2
     float dx;
     float2 *F2;             // R^3 out (k-space data, F/C/dx)
-    float2 *G;              // R^3 out (F2 after the z inverse transform)
+    float2 *G;              // R^3 out (F2 after the z inverse transform, times g_scale)
+    float g_scale;
     uint32_t *counts;       // optional R^3 hit counts
     uint8_t *mask;          // optional R^3 hit mask (1 where counts > 0)
+    int *active;            // optional: active-tile header to clear for pack_measured
     // frequency interpolation between scan angles (FI mapping) when fi_theta is set:
     // fi_theta = the A scan angles ascending (rad), fi_frame = the frame of each
     const double *fi_theta;
@@ -50,8 +52,9 @@ struct LoopArgs {
     const uint8_t *mask;
     float2 *out;            // final RI volume (octant shifted), only for the final pass
     int R;
-    float inv_n3, k2, n_med, n_med2;
-    float s1;   // -1 / (R^3 k^2)
+    float k2, n_med, n_med2;
+    float s1;   // -1 / (R^2 k^2) on the plane scheme, -1 / (R k^2) on the line passes
+    float inv_r;   // 1 / R: the z passes (and the y inverse pass) leave normalised lines
     float s2;   // -k^2 / n_med^2
     int *err;   // device status word: a bounded wait that ran out records a nonzero code
     int staged; // z pass: F2 / mask tiles staged by TMA (set by the launcher)
@@ -64,6 +67,9 @@ struct LoopArgs {
     const int *tprefix;     // tprefix[tile * R + z]: kept samples of the tile before row z
     const float2 *tvals;
     int packed;
+    // tiles with at least one kept sample: ztiles[0 .. *zcount), and per 8 columns x of
+    // the volume whether any tile over them has one (xactive; NULL: every column)
+    const int *ztiles, *zcount, *xactive;
     // accelerated loop (projected FISTA): the pass that applies est_n and modify keeps
     // the projected iterate x_k in xprev and sends w_k = x_k + beta (x_k - x_{k-1}) on
     // to the forward transform; xprev == nullptr: the plain loop
@@ -72,9 +78,21 @@ struct LoopArgs {
 };
 
 // Packs F2 (mode 0: re != 0 && im != 0; mode 1: mask != 0) into per-tile masks,
-// counts, row prefixes and values for the z pass (TB lines per tile, 8, 16 or 32).
+// counts, row prefixes and values for the z pass (TB lines per tile, 8, 16 or 32), and
+// lists the tiles that keep a sample: active holds a header {count, 3 unused, R / 8
+// column flags}, zero before the call, and the tile list (active_ints(R) entries, enough
+// for every TB; active_view points a pass at them).  active may be NULL for sides whose
+// passes take every tile (skip_empty_tiles, loop_passes.cuh).
 cudaError_t pack_measured(const float2 *F2, const uint8_t *mask, int R, int TB, uint32_t *tmask, int *tcount,
-                          int *tprefix, float2 *tvals, cudaStream_t s);
+                          int *tprefix, float2 *tvals, int *active, cudaStream_t s);
+__host__ __device__ inline int active_head(int R) { return 4 + R / 8; }
+inline size_t active_ints(int R) { return active_head(R) + (size_t)R * R / 8; }
+inline void active_view(LoopArgs &a, const int *active, int R)
+{
+    a.zcount = active;
+    a.xactive = active + 4;
+    a.ztiles = active + active_head(R);
+}
 
 cudaError_t launch_ewald(const EwaldArgs &a, cudaStream_t s);
 cudaError_t launch_xpass(const LoopArgs &a, bool final_pass, cudaStream_t s);
@@ -152,6 +170,9 @@ cudaError_t pocs_finish(const PocsBufs &b, float n_med, float2 *ri, cudaStream_t
 cudaError_t fft_rows(float2 *data, int L, long nlines, bool inverse, cudaStream_t s);
 cudaError_t fft_cols(float2 *data, int L, long nlines, int nx, long plane, long ld, bool inverse,
                      cudaStream_t s);
+// cols from src to dst (which may be the same buffer), the result scaled.
+cudaError_t fft_cols_from(const float2 *src, float2 *dst, int L, long nlines, int nx, long plane, long ld,
+                          bool inverse, float scale, cudaStream_t s);
 // 3-D transform in place (cuFFT3D semantics: inverse scaled by 1/(R^3)).
 cudaError_t fft3d(float2 *data, int R, bool inverse, cudaStream_t s);
 cudaError_t scale_complex(float2 *data, long n, float s, bool conjugate, cudaStream_t st);

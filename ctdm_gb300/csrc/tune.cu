@@ -204,19 +204,29 @@ cudaError_t autotune_loop(int R, int check_mode, int *chosen, double *ms_out, in
     if (e == cudaSuccess) e = cudaMalloc(&F2, sizeof(float2) * r3);
     if (e == cudaSuccess && check_mode) e = cudaMalloc(&mask, r3);
     if (e == cudaSuccess) e = cudaMalloc(&err, sizeof(int));
-    // packed z passes are timed as the loop runs them, on empty tiles (no measured
-    // samples: the same transforms, loads and stores, none of the few value loads)
+    // packed z passes are timed with every tile listed and no sample kept in any (the
+    // same transforms, loads and stores as an active tile, none of the few value loads)
     int tbmin = 0;
     for (int v = 0; v < nv; v++) {
         const int tb = ztile_of(R, v);
         if (tb > 0 && (tbmin == 0 || tb < tbmin)) tbmin = tb;
     }
     uint32_t *tmask = nullptr;
-    int *tcount = nullptr, *tprefix = nullptr;
+    int *tcount = nullptr, *tprefix = nullptr, *active = nullptr;
     const size_t tiles = tbmin ? (size_t)R * R / tbmin : 0;
     if (e == cudaSuccess && tiles) e = cudaMalloc(&tmask, sizeof(uint32_t) * tiles * R);
     if (e == cudaSuccess && tiles) e = cudaMalloc(&tcount, sizeof(int) * tiles);
     if (e == cudaSuccess && tiles) e = cudaMalloc(&tprefix, sizeof(int) * tiles * R);
+    // active[4 v]: tile count of variant v; then the column flags and the tile list
+    std::vector<int> hact;
+    if (tiles) {
+        hact.assign(16 + R / 8, 1);
+        for (int v = 0; v < nv && v < 4; v++) hact[4 * v] = ztile_of(R, v) > 0 ? R * R / ztile_of(R, v) : 0;
+        for (size_t i = 0; i < tiles; i++) hact.push_back((int)i);
+    }
+    if (e == cudaSuccess && tiles) e = cudaMalloc(&active, sizeof(int) * hact.size());
+    if (e == cudaSuccess && tiles)
+        e = cudaMemcpy(active, hact.data(), sizeof(int) * hact.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
     if (e == cudaSuccess && tiles) e = cudaMemsetAsync(tmask, 0, sizeof(uint32_t) * tiles * R, s);
     if (e == cudaSuccess && tiles) e = cudaMemsetAsync(tcount, 0, sizeof(int) * tiles, s);
@@ -234,7 +244,7 @@ cudaError_t autotune_loop(int R, int check_mode, int *chosen, double *ms_out, in
         a.out = F2;   // the final x pass is not timed
         a.R = R;
         const double k2 = 1.0e14, nm = 1.337;
-        a.inv_n3 = (float)(1.0 / (double)r3);
+        a.inv_r = (float)(1.0 / R);
         a.k2 = (float)k2;
         a.n_med = (float)nm;
         a.n_med2 = (float)(nm * nm);
@@ -249,6 +259,8 @@ cudaError_t autotune_loop(int R, int check_mode, int *chosen, double *ms_out, in
         auto zargs = [&](int v) {
             LoopArgs z = a;
             z.packed = tiles && ztile_of(R, v) > 0 ? 1 : 0;
+            z.zcount = active + 4 * v;
+            z.ztiles = active + 16 + R / 8;
             return z;
         };
         const int kinds[3] = {LOOP_X, LOOP_Y_FWD, LOOP_Z};
@@ -308,6 +320,7 @@ cudaError_t autotune_loop(int R, int check_mode, int *chosen, double *ms_out, in
     cudaFree(tmask);
     cudaFree(tcount);
     cudaFree(tprefix);
+    cudaFree(active);
     if (e != cudaSuccess) return e;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
