@@ -12,6 +12,7 @@
 
 #include "fft_line.cuh"
 #include "kernels.cuh"
+#include "line_kernels.cuh"
 #include "point_ops.cuh"
 #include "tma.cuh"
 
@@ -55,106 +56,58 @@ namespace ctdm {
 
 using fftl::Plan;
 
-// ------------------------------------------------------------ load / store
-// Contiguous lines: line l occupies data[l*L .. l*L+L).
+// ------------------------------------------------------------ generic passes
+// Plan of the strided lines: 16 lines (128-byte segments) and at most 24 points per thread
+// where the length allows (more warps to hide the loads behind): 181 x 512 columns of 512,
+// 229 -> 181 us per launch against 32 points per thread; z lines of 384^3, 244 -> 224 us
+// against 48.
 template <int L>
-__device__ __forceinline__ void load_rows(float2 *buf, const float2 *__restrict__ src, long line0, long nlines)
-{
-    using P = Plan<L>;
-    const float4 *s4 = reinterpret_cast<const float4 *>(src);
-#pragma unroll 4
-    for (int e = threadIdx.x; e < P::B * L / 2; e += P::THREADS) {
-        const int b = (2 * e) / L, p = 2 * e - b * L;
-        const long l = line0 + b;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (l < nlines) v = __ldcs(&s4[(l * L + p) / 2]);
-        buf[b * P::LP + p] = make_float2(v.x, v.y);
-        buf[b * P::LP + p + 1] = make_float2(v.z, v.w);
-    }
-}
-
-template <int L>
-__device__ __forceinline__ void store_rows(float2 *dst, const float2 *buf, long line0, long nlines)
-{
-    using P = Plan<L>;
-    float4 *d4 = reinterpret_cast<float4 *>(dst);
-#pragma unroll 4
-    for (int e = threadIdx.x; e < P::B * L / 2; e += P::THREADS) {
-        const int b = (2 * e) / L, p = 2 * e - b * L;
-        const long l = line0 + b;
-        if (l < nlines) {
-            float2 a = buf[b * P::LP + p], c = buf[b * P::LP + p + 1];
-            __stcs(&d4[(l * L + p) / 2], make_float4(a.x, a.y, c.x, c.y));
-        }
-    }
-}
+struct ColPlan : Plan<L> {};
+template <> struct ColPlan<384> : fftl::PV<384, 1> {};
+template <> struct ColPlan<512> : fftl::PV<512, 1> {};
+template <> struct ColPlan<768> : fftl::PV<768, 2> {};
 
 // Strided lines: element p of line l at (l % nx) + (l / nx) * plane + p * ld.
 // Threads are b-fastest so B consecutive lines give coalesced segments.
 template <int L>
 __device__ __forceinline__ long col_base(long line0, int nx, long plane, long nlines, bool &ok)
 {
-    using P = Plan<L>;
+    using P = ColPlan<L>;
     const int b = threadIdx.x % P::B;
     const long l = line0 + b;
     ok = l < nlines;
     return (l % nx) + (l / nx) * plane;
 }
 
-template <int L>
-__device__ __forceinline__ void load_cols(float2 *buf, const float2 *__restrict__ src, long base, bool ok, long ld)
-{
-    using P = Plan<L>;
-    const int b = threadIdx.x % P::B, t = threadIdx.x / P::B;
-#pragma unroll 4
-    for (int p = t; p < L; p += P::T) buf[b * P::LP + p] = ok ? __ldcs(&src[base + p * ld]) : make_float2(0.f, 0.f);
-}
-
-template <int L>
-__device__ __forceinline__ void store_cols(float2 *dst, const float2 *buf, long base, bool ok, long ld)
-{
-    using P = Plan<L>;
-    const int b = threadIdx.x % P::B, t = threadIdx.x / P::B;
-    if (!ok) return;
-#pragma unroll 4
-    for (int p = t; p < L; p += P::T) __stcs(&dst[base + p * ld], buf[b * P::LP + p]);
-}
-
-// ------------------------------------------------------------ generic passes
+// src may be data itself (in place); the result is scaled by `scale`.  xactive (y lines of
+// a volume, B <= nx): columns whose flags are all 0 are left as they are.
 template <int L, bool INV>
-__global__ void __launch_bounds__(Plan<L>::THREADS) rows_kernel(float2 *data, const float2 *__restrict__ tw, long nlines)
+__global__ void __launch_bounds__(ColPlan<L>::THREADS) cols_kernel(const float2 *src, float2 *data,
+                                                                   const float2 *__restrict__ tw, long nlines, int nx,
+                                                                   long plane, long ld, float scale,
+                                                                   const int *__restrict__ xactive)
 {
-    extern __shared__ float4 smem4[];
-    float2 *buf = reinterpret_cast<float2 *>(smem4);
-    const long line0 = (long)blockIdx.x * Plan<L>::B;
-    load_rows<L>(buf, data, line0, nlines);
-    __syncthreads();
-    Plan<L>::template run<INV>(buf, tw);
-    store_rows<L>(data, buf, line0, nlines);
-}
-
-// src may be data itself (in place); the result is scaled by `scale`.
-template <int L, bool INV>
-__global__ void __launch_bounds__(Plan<L>::THREADS) cols_kernel(const float2 *src, float2 *data, const float2 *__restrict__ tw,
-                                                                long nlines, int nx, long plane, long ld, float scale)
-{
-    using P = Plan<L>;
-    using En = fftl::Ends<L>;
+    using P = ColPlan<L>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
     const long line0 = (long)blockIdx.x * P::B;
+    if (xactive) {
+        int any = 0;
+        for (int x = 0; x < (P::B < nx ? P::B : nx); x += 8) any |= __ldg(&xactive[(line0 % nx + x) / 8]);
+        if (!any) return;
+    }
     bool ok;
     const long base = col_base<L>(line0, nx, plane, nlines, ok);
     const int t = threadIdx.x / P::B;
     float2 v[P::E];
 #pragma unroll
     for (int i = 0; i < P::E; i++)
-        v[i] = ok ? __ldcs(&src[base + (long)fftl::slot_pos<L, P::T, En::F>(i, t) * ld]) : make_float2(0.f, 0.f);
+        v[i] = ok ? __ldcs(&src[base + (long)fftl::slot_pos<L, P::T, P::F0>(i, t) * ld]) : make_float2(0.f, 0.f);
     P::template seq<INV, false, false>(buf, v, tw);
     if (!ok) return;
 #pragma unroll
     for (int i = 0; i < P::E; i++)
-        __stcs(&data[base + (long)fftl::slot_pos<L, P::T, En::Rv>(i, t) * ld], cscale(v[i], scale));
+        __stcs(&data[base + (long)fftl::slot_pos<L, P::T, P::RV0>(i, t) * ld], cscale(v[i], scale));
 }
 
 // Large dynamic shared memory opt-in and the largest shared-memory carveout, so
@@ -172,35 +125,36 @@ static cudaError_t prep_launch(K kernel, size_t smem)
 }
 
 template <int L>
-static cudaError_t rows_launch(float2 *data, long nlines, bool inv, cudaStream_t s)
+static cudaError_t rows_launch(const float2 *src, float2 *dst, long nlines, bool inv, float scale, cudaStream_t s)
 {
-    using P = Plan<L>;
-    const size_t smem = fftl::smem_bytes<L>();
-    const long grid = (nlines + P::B - 1) / P::B;
-    auto k = inv ? rows_kernel<L, true> : rows_kernel<L, false>;
-    cudaError_t e = prep_launch<L>(k, smem);
-    if (e != cudaSuccess) return e;
-    k<<<(unsigned)grid, P::THREADS, smem, s>>>(data, twiddles(L), nlines); note_launch();
-    return cudaGetLastError();
+    const LoadComplex ld = {src};
+    const StoreScaled st = {dst, scale};
+    return inv ? rows_fn_launch<RowPlan<L>, true>(ld, st, nlines, s) : rows_fn_launch<RowPlan<L>, false>(ld, st, nlines, s);
 }
 
 template <int L>
 static cudaError_t cols_launch(const float2 *src, float2 *data, long nlines, int nx, long plane, long ld, bool inv,
-                               float scale, cudaStream_t s)
+                               float scale, const int *xactive, cudaStream_t s)
 {
-    using P = Plan<L>;
-    const size_t smem = fftl::smem_bytes<L>();
+    using P = ColPlan<L>;
+    const size_t smem = fftl::plan_smem<P>();
     const long grid = (nlines + P::B - 1) / P::B;
     auto k = inv ? cols_kernel<L, true> : cols_kernel<L, false>;
     cudaError_t e = prep_launch<L>(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<(unsigned)grid, P::THREADS, smem, s>>>(src, data, twiddles(L), nlines, nx, plane, ld, scale); note_launch();
+    k<<<(unsigned)grid, P::THREADS, smem, s>>>(src, data, twiddles(L), nlines, nx, plane, ld, scale, xactive); note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t fft_rows(float2 *data, int L, long nlines, bool inverse, cudaStream_t s)
 {
-    CTDM_DISPATCH_L(L, rows_launch, data, nlines, inverse, s)
+    return fft_rows_from(data, data, L, nlines, inverse, 1.0f, s);
+}
+
+cudaError_t fft_rows_from(const float2 *src, float2 *dst, int L, long nlines, bool inverse, float scale,
+                          cudaStream_t s)
+{
+    CTDM_DISPATCH_L(L, rows_launch, src, dst, nlines, inverse, scale, s)
 }
 
 cudaError_t fft_cols(float2 *data, int L, long nlines, int nx, long plane, long ld, bool inverse, cudaStream_t s)
@@ -209,9 +163,9 @@ cudaError_t fft_cols(float2 *data, int L, long nlines, int nx, long plane, long 
 }
 
 cudaError_t fft_cols_from(const float2 *src, float2 *dst, int L, long nlines, int nx, long plane, long ld,
-                          bool inverse, float scale, cudaStream_t s)
+                          bool inverse, float scale, cudaStream_t s, const int *xactive)
 {
-    CTDM_DISPATCH_L(L, cols_launch, src, dst, nlines, nx, plane, ld, inverse, scale, s)
+    CTDM_DISPATCH_L(L, cols_launch, src, dst, nlines, nx, plane, ld, inverse, scale, xactive, s)
 }
 
 __global__ void scale_kernel(float2 *d, long n, float s, bool conj)
@@ -487,6 +441,7 @@ __global__ void __launch_bounds__(256) pack_measured_kernel(const float2 *__rest
     }
     __syncthreads();
     for (int z = threadIdx.x; z < R; z += 256) tprefix[tile * R + z] = spre[z];
+    if (!tvals) return;
     float2 *tv = tvals + tile * (long)TB * R;
     const uint32_t below = (1u << b) - 1u;
     for (int z0 = 0; z0 < R; z0 += ZR) {

@@ -82,7 +82,8 @@ struct LoopArgs {
 // lists the tiles that keep a sample: active holds a header {count, 3 unused, R / 8
 // column flags}, zero before the call, and the tile list (active_ints(R) entries, enough
 // for every TB; active_view points a pass at them).  active may be NULL for sides whose
-// passes take every tile (skip_empty_tiles, loop_passes.cuh).
+// passes take every tile (skip_empty_tiles, loop_passes.cuh), tvals where the values are
+// kept elsewhere.
 cudaError_t pack_measured(const float2 *F2, const uint8_t *mask, int R, int TB, uint32_t *tmask, int *tcount,
                           int *tprefix, float2 *tvals, int *active, cudaStream_t s);
 __host__ __device__ inline int active_head(int R) { return 4 + R / 8; }
@@ -170,9 +171,12 @@ cudaError_t pocs_finish(const PocsBufs &b, float n_med, float2 *ri, cudaStream_t
 cudaError_t fft_rows(float2 *data, int L, long nlines, bool inverse, cudaStream_t s);
 cudaError_t fft_cols(float2 *data, int L, long nlines, int nx, long plane, long ld, bool inverse,
                      cudaStream_t s);
-// cols from src to dst (which may be the same buffer), the result scaled.
+// rows / cols from src to dst (which may be the same buffer), the result scaled; xactive
+// (y lines of a volume): per 8 columns x, 0 leaves the columns out.
+cudaError_t fft_rows_from(const float2 *src, float2 *dst, int L, long nlines, bool inverse, float scale,
+                          cudaStream_t s);
 cudaError_t fft_cols_from(const float2 *src, float2 *dst, int L, long nlines, int nx, long plane, long ld,
-                          bool inverse, float scale, cudaStream_t s);
+                          bool inverse, float scale, cudaStream_t s, const int *xactive = nullptr);
 // 3-D transform in place (cuFFT3D semantics: inverse scaled by 1/(R^3)).
 cudaError_t fft3d(float2 *data, int R, bool inverse, cudaStream_t s);
 cudaError_t scale_complex(float2 *data, long n, float s, bool conjugate, cudaStream_t st);
