@@ -26,6 +26,17 @@ __device__ __forceinline__ float2 cmul_mi(float2 a)
     return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
+// The same pointer, opaque to the compiler: table loads through it stay where they are
+// written.  In a loop over line batches every thread's twiddles are loop-invariant, and
+// keeping them in registers across the loop (15 complex values per radix-16 stage) costs
+// more than reloading them from L1.
+template <class T>
+__device__ __forceinline__ const T *fresh(const T *p)
+{
+    asm volatile("" : "+l"(p));
+    return p;
+}
+
 __device__ __forceinline__ int imod(int a, int b)
 {
     int r = a % b;

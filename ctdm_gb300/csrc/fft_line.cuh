@@ -281,6 +281,12 @@ struct PlanT<L_, B_, T_, Radices<FW...>, Radices<RV...>> {
     {
         stages<L, T, LP, INV, false, false, true, 1, FW...>(buf, v, tw, threadIdx.x / T, threadIdx.x % T);
     }
+    // seq_row with its first stage read from shared memory
+    template <bool INV>
+    __device__ static __forceinline__ void seq_row_from(float2 *buf, float2 *v, const float2 *tw)
+    {
+        stages<L, T, LP, INV, true, false, true, 1, FW...>(buf, v, tw, threadIdx.x / T, threadIdx.x % T);
+    }
     template <bool INV>
     __device__ static __forceinline__ void seqr_row(float2 *buf, float2 *v, const float2 *tw)
     {

@@ -36,12 +36,12 @@ constexpr long kScratchFloats = 4194304;
 constexpr int kMinM = 16, kMaxM = 256;
 static_assert(kMinM << (5 - 1) == kMaxM, "five sides, 16 to 256");
 constexpr int kSides = 5;                     // 16, 32, 64, 128, 256
-constexpr int kTwTotal = 32 + 64 + 128 + 256 + 512;          // FFT tables of length 2M
+constexpr int kTwTotal = 16 + 32 + 64 + 128 + 256;           // FFT tables of length M
 constexpr int kDctTotal = 33 + 65 + 129 + 257 + 513;         // cos/sin(k pi / 2M), k = 0..2M
 constexpr int kEigTotal = 16 + 32 + 64 + 128 + 256;          // 4 sin^2(2 pi k / (4M - 1))
 
-// Scratch: the row-transformed map between the three passes.  Every element a
-// pass reads was written by the previous pass of the same call, so it needs no
+// Scratch: the transformed map between the three phases.  Every element a
+// phase reads was written by the previous one of the same call, so it needs no
 // clearing; it keeps the last call's contents.
 static __device__ __align__(256) float g_noalloc_scratch[kScratchFloats];
 static __device__ __align__(256) float2 g_noalloc_tw[kTwTotal];
@@ -76,7 +76,7 @@ void offsets(int idx, int &tw, int &dct, int &eig)
 {
     tw = dct = eig = 0;
     for (int i = 0, m = kMinM; i < idx; i++, m *= 2) {
-        tw += 2 * m;
+        tw += m;
         dct += 2 * m + 1;
         eig += m;
     }
@@ -103,12 +103,11 @@ cudaError_t setup_current_device(DeviceSymbols *&out)
         for (int i = 0, m = kMinM; i < kSides; i++, m *= 2) {
             int otw, odct, oeig;
             offsets(i, otw, odct, oeig);
-            const int L = 2 * m;
-            for (int k = 0; k < L; k++) {
-                const double a = -2.0 * pi * (double)k / (double)L;
+            for (int k = 0; k < m; k++) {
+                const double a = -2.0 * pi * (double)k / (double)m;
                 tw[otw + k] = make_float2((float)cos(a), (float)sin(a));
             }
-            for (int k = 0; k <= L; k++) {
+            for (int k = 0; k <= 2 * m; k++) {
                 const double a = (double)k * pi / (2.0 * m);
                 dct[odct + k] = make_float2((float)cos(a), (float)sin(a));
             }
