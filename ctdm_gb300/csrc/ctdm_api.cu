@@ -262,6 +262,7 @@ struct ctdm_ctx {
     } *pin = nullptr;
     cudaEvent_t geom_done = nullptr, carrier_done = nullptr;
     bool carrier_pending = false;
+    float fz0_lo = 0.f, fz0_hi = 0.f;   // upload_geometry's angles: range of fz0 / df
     // host-buffer uploads: a copy stream and one event per chunk of angles
     static const int kChunks = 16;
     cudaStream_t copy = nullptr;
@@ -566,6 +567,14 @@ static ctdm_status upload_geometry(ctdm_ctx *c, const float *angx, const float *
 {
     std::vector<AngleGeom> g;
     angle_geometry(angx, angy, A, fm0, df, g);
+    c->fz0_lo = c->fz0_hi = 0.f;
+    bool any = false;
+    for (const AngleGeom &q : g) {
+        if (!q.valid) continue;
+        c->fz0_lo = any ? std::min(c->fz0_lo, q.fz0s) : q.fz0s;
+        c->fz0_hi = any ? std::max(c->fz0_hi, q.fz0s) : q.fz0s;
+        any = true;
+    }
     CK(ensure(c, B_GEOM, sizeof(AngleGeom) * A), "alloc geometry");
     if (A <= (int)(sizeof c->pin->geom / sizeof(AngleGeom))) {
         // pinned staging: the previous call's copy has left it once geom_done fired
@@ -1432,7 +1441,6 @@ extern "C" ctdm_status ctdm_map_ewald(ctdm_ctx *c, int A, int R, const ctdm_cflo
     const long r3 = (long)R * R * R;
     ctdm_status st = upload_geometry(c, h_angx, h_angy, A, fm0, df, s);
     if (st != CTDM_OK) return st;
-    CK(ensure(c, B_TMP, sizeof(float2) * r3), "alloc G");
     EwaldArgs ea = {};
     ea.U = reinterpret_cast<const float2 *>(d_U);
     ea.geom = B<AngleGeom>(c, B_GEOM);
@@ -1443,8 +1451,9 @@ extern "C" ctdm_status ctdm_map_ewald(ctdm_ctx *c, int A, int R, const ctdm_cflo
     ea.fm02 = fm0 * fm0;
     ea.fm02s = (float)((fm0 / df) * (fm0 / df));
     ea.dx = (float)dx;
+    ea.fz0_lo = c->fz0_lo;
+    ea.fz0_hi = c->fz0_hi;
     ea.F2 = reinterpret_cast<float2 *>(d_F2);
-    ea.G = B<float2>(c, B_TMP);
     ea.counts = d_counts;
     ea.mask = nullptr;
     CK(launch_ewald(ea, s), "ewald mapping");
@@ -1482,7 +1491,6 @@ extern "C" ctdm_status ctdm_map_fi(ctdm_ctx *c, int A, int R, const ctdm_cfloat 
     }
     CK(ensure(c, B_FIT, tab.size()), "alloc FI tables");
     CK(cudaMemcpyAsync(c->buf[B_FIT], tab.data(), tab.size(), cudaMemcpyHostToDevice, s), "upload FI tables");
-    CK(ensure(c, B_TMP, sizeof(float2) * r3), "alloc G");
     EwaldArgs ea = {};
     ea.U = reinterpret_cast<const float2 *>(d_U);
     ea.geom = B<AngleGeom>(c, B_GEOM);
@@ -1493,8 +1501,9 @@ extern "C" ctdm_status ctdm_map_fi(ctdm_ctx *c, int A, int R, const ctdm_cfloat 
     ea.fm02 = fm0 * fm0;
     ea.fm02s = (float)((fm0 / df) * (fm0 / df));
     ea.dx = (float)dx;
+    ea.fz0_lo = c->fz0_lo;
+    ea.fz0_hi = c->fz0_hi;
     ea.F2 = reinterpret_cast<float2 *>(d_F2);
-    ea.G = B<float2>(c, B_TMP);
     ea.counts = d_counts;
     ea.fi_theta = B<double>(c, B_FIT);
     ea.fi_frame = reinterpret_cast<const int *>(B<double>(c, B_FIT) + A);

@@ -32,10 +32,11 @@ struct EwaldArgs {
     const AngleGeom *geom;  // A entries
     int A, R;
     double fm0, df, fm02;
+    float fz0_lo, fz0_hi;   // range of fz0 / df over the angles (both 0: not known)
     float fm02s;            // (fm0/df)^2
     float dx;
     float2 *F2;             // R^3 out (k-space data, F/C/dx)
-    float2 *G;              // R^3 out (F2 after the z inverse transform, times g_scale)
+    float2 *G;              // optional R^3 out (F2 after the z inverse transform, times g_scale)
     float g_scale;
     uint32_t *counts;       // optional R^3 hit counts
     uint8_t *mask;          // optional R^3 hit mask (1 where counts > 0)
