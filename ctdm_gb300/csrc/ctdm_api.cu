@@ -672,6 +672,9 @@ static ctdm_status do_qpi(ctdm_ctx *c, int N, int M, int A, const float *holo, c
     return qpi_angles(c, N, M, A, 0, A, holo, 4, bg_per_angle, phase, amp, s);
 }
 
+// Scale of the z lines that the loop starts from.
+static float loop_g_scale(int R) { return skip_empty_tiles(R) ? (float)(1.0 / R) : 1.0f; }
+
 // The positivity loop (BatchRecon, cTDM/HilbertTransform.cu:1943-2004), or with
 // accelerated = 1 the same projection step with Nesterov momentum (projected FISTA
 // with the data-replacement step, no regulariser): the pass that applies est_n and
@@ -707,7 +710,7 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
         CK(ensure(c, B_TPRE, sizeof(int) * tiles * R), "alloc packed prefixes");
         CK(ensure(c, B_TVALS, sizeof(float2) * r3), "alloc packed values");
         CK(pack_measured(F2, check_mode == CTDM_CHECK_MASK ? mask : nullptr, R, TB, B<uint32_t>(c, B_TMASK),
-                         B<int>(c, B_TCOUNT), B<int>(c, B_TPRE), B<float2>(c, B_TVALS), R > 128 ? B<int>(c, B_TACT) : nullptr, s),
+                         B<int>(c, B_TCOUNT), B<int>(c, B_TPRE), B<float2>(c, B_TVALS), skip_empty_tiles(R) ? B<int>(c, B_TACT) : nullptr, s),
            "pack measured samples");
         la.tmask = B<uint32_t>(c, B_TMASK);
         la.tcount = B<int>(c, B_TCOUNT);
@@ -729,10 +732,10 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
         t_k = t_n;
     };
     StageTimer &tm = c->timer;
-    // G holds z lines normalised by 1 / R (g_scale of the mapping, the z passes); the y
-    // inverse line pass normalises too, the plane pass leaves 1 / R^2 to s1
+    // where empty tiles are skipped G holds z lines normalised by 1 / R (loop_g_scale, the z
+    // passes) and the y inverse line pass normalises too; the rest is left to s1
     const bool planes = loop_scheme(R) >= 1;
-    la.s1 = (float)(-1.0 / ((planes ? (double)R * R : (double)R) * k2));
+    la.s1 = (float)(-1.0 / ((!skip_empty_tiles(R) ? (double)R * R * R : planes ? (double)R * R : (double)R) * k2));
     if (planes) {
         // plane + z passes, 8- or 4-CTA clusters per plane (schemes 1, 2; the plane pass
         // records under the x-pass stage)
@@ -982,7 +985,7 @@ static ctdm_status pipeline_core(ctdm_ctx *c, const ctdm_params *p, int A, int M
     ea.dx = (float)p->dx;
     ea.F2 = B<float2>(c, B_F2);
     ea.G = B<float2>(c, B_G);
-    ea.g_scale = (float)(1.0 / R);
+    ea.g_scale = loop_g_scale(R);
     ea.counts = mask_mode ? B<uint32_t>(c, B_COUNTS) : nullptr;
     ea.mask = mask_mode ? B<uint8_t>(c, B_MASK) : nullptr;
     ea.active = B<int>(c, B_TACT);
@@ -1564,7 +1567,23 @@ extern "C" ctdm_status ctdm_pocs(ctdm_ctx *c, int R, const ctdm_pocs_params *p, 
     b.g2 = B<float>(c, B_PG2);
     b.Vp = B<float>(c, B_PVP);
     b.G = B<float2>(c, B_G);
-    b.F2 = reinterpret_cast<const float2 *>(d_F2);
+    const int TB = pocs_tile(R);
+    const size_t tiles = (size_t)R * R / TB;
+    CK(ensure(c, B_TMASK, sizeof(uint32_t) * tiles * R), "alloc packed masks");
+    CK(ensure(c, B_TCOUNT, sizeof(int) * tiles), "alloc packed counts");
+    CK(ensure(c, B_TPRE, sizeof(int) * tiles * R), "alloc packed prefixes");
+    CK(ensure(c, B_TVALS, sizeof(float2) * r3), "alloc packed values");
+    CK(ensure(c, B_TACT, sizeof(int) * active_ints(R)), "alloc active tiles");
+    CK(cudaMemsetAsync(c->buf[B_TACT], 0, sizeof(int) * active_head(R), s), "clear active tiles");
+    CK(pack_measured(reinterpret_cast<const float2 *>(d_F2), nullptr, R, TB, B<uint32_t>(c, B_TMASK),
+                     B<int>(c, B_TCOUNT), B<int>(c, B_TPRE), B<float2>(c, B_TVALS), B<int>(c, B_TACT), s,
+                     PACK_NONZERO),
+       "pack measured samples");
+    b.tmask = B<uint32_t>(c, B_TMASK);
+    b.tcount = B<int>(c, B_TCOUNT);
+    b.tprefix = B<int>(c, B_TPRE);
+    b.tvals = B<float2>(c, B_TVALS);
+    b.active = B<int>(c, B_TACT);
     b.part = B<double>(c, B_PPART);
     b.ctl = B<PocsCtl>(c, B_PCTL);
     b.hist = B<double>(c, B_PHIST);
@@ -1573,7 +1592,6 @@ extern "C" ctdm_status ctdm_pocs(ctdm_ctx *c, int R, const ctdm_pocs_params *p, 
     b.tv_eps = (float)p->tv_eps;
     CK(cudaMemcpyAsync(b.ctl, &ctl, sizeof ctl, cudaMemcpyHostToDevice, s), "upload controller");
     CK(cudaMemsetAsync(b.V, 0, sizeof(float) * r3, s), "zero V");
-    CK(cudaMemsetAsync(b.G, 0, sizeof(float2) * r3, s), "zero G");
     for (int it = 0; it < p->iterations; it++) CK(pocs_iteration(b, p->tv_steps, want_dd, s), "POCS iteration");
     CK(pocs_finish(b, (float)n_med, reinterpret_cast<float2 *>(d_ri), s), "POCS output");
     if (h_hist && p->iterations > 0) {
@@ -1611,7 +1629,7 @@ extern "C" ctdm_status ctdm_positivity_ex(ctdm_ctx *c, int R, int iterations, in
     const long rr = (long)R * R, r3 = rr * R;
     CK(ensure(c, B_G, sizeof(float2) * r3), "alloc G");
     float2 *G = B<float2>(c, B_G);
-    CK(fft_cols_from(reinterpret_cast<const float2 *>(d_F2), G, R, rr, (int)rr, 0, rr, true, (float)(1.0 / R), s),
+    CK(fft_cols_from(reinterpret_cast<const float2 *>(d_F2), G, R, rr, (int)rr, 0, rr, true, loop_g_scale(R), s),
        "z inverse");
     CK(ensure(c, B_TACT, sizeof(int) * active_ints(R)), "alloc active tiles");
     CK(cudaMemsetAsync(c->buf[B_TACT], 0, sizeof(int) * active_head(R), s), "clear active tiles");

@@ -25,6 +25,7 @@
 // the TV step reads its size from there, the reductions' last blocks update it.  An
 // iteration is therefore a fixed launch sequence that a CUDA graph can replay.
 #include "kernels.cuh"
+#include "line_kernels.cuh"
 #include "point_ops.cuh"
 
 namespace ctdm {
@@ -40,26 +41,28 @@ __device__ __forceinline__ double warp_sum(double v)
 }
 
 // Block sum of v in a fixed order; the result is valid in thread 0.
+template <int NT>
 __device__ double block_sum(double v)
 {
-    __shared__ double sw[kThreads / 32];
+    __shared__ double sw[NT / 32];
     v = warp_sum(v);
     const int w = threadIdx.x >> 5;
     if ((threadIdx.x & 31) == 0) sw[w] = v;
     __syncthreads();
     double t = 0.0;
     if (threadIdx.x == 0)
-        for (int i = 0; i < kThreads / 32; i++) t += sw[i];
+        for (int i = 0; i < NT / 32; i++) t += sw[i];
     __syncthreads();
     return t;
 }
 
 // Writes this block's partial; the last block to finish sums all partials in index
 // order and returns true in its thread 0 with *total set.
+template <int NT = kThreads>
 __device__ bool grid_sum(double v, double *part, unsigned *ticket, double *total)
 {
     __shared__ bool last;
-    const double b = block_sum(v);
+    const double b = block_sum<NT>(v);
     if (threadIdx.x == 0) {
         part[blockIdx.x] = b;
         __threadfence();
@@ -71,14 +74,14 @@ __device__ bool grid_sum(double v, double *part, unsigned *ticket, double *total
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;   // four chains: the loads overlap
     const int n = (int)gridDim.x;
     int i = threadIdx.x;
-    for (; i + 3 * kThreads < n; i += 4 * kThreads) {
+    for (; i + 3 * NT < n; i += 4 * NT) {
         s0 += __ldcg(&part[i]);
-        s1 += __ldcg(&part[i + kThreads]);
-        s2 += __ldcg(&part[i + 2 * kThreads]);
-        s3 += __ldcg(&part[i + 3 * kThreads]);
+        s1 += __ldcg(&part[i + NT]);
+        s2 += __ldcg(&part[i + 2 * NT]);
+        s3 += __ldcg(&part[i + 3 * NT]);
     }
-    for (; i < n; i += kThreads) s0 += __ldcg(&part[i]);
-    double s = block_sum((s0 + s1) + (s2 + s3));
+    for (; i < n; i += NT) s0 += __ldcg(&part[i]);
+    double s = block_sum<NT>((s0 + s1) + (s2 + s3));
     if (threadIdx.x == 0) {
         *total = s;
         *ticket = 0u;
@@ -101,76 +104,137 @@ __device__ __forceinline__ float re_sqrt1p_m1(float2 v)
 // thread issues its kPer loads before it uses any of them (R^3 is a multiple of 1024).
 constexpr int kPer = 4;
 
-__global__ void __launch_bounds__(kThreads) dc_kernel(float2 *G, const float2 *__restrict__ F2, long n,
-                                                      const PocsCtl *__restrict__ ctl, float y_scale)
+// ---- the data step's transforms with the work between them
+// FFT_x reads the real volume V (LoadReal), FFT_y and the z lines follow; the z line kernel
+// replaces the measured samples (packed per tile) and transforms back; IFFT_y; and IFFT_x
+// hands its rows to the projection (or the output).  Tiles and y lines without a measured
+// sample are left out: there the transforms cancel, the z and y inverses being normalised.
+// At 256^3 (line scan of 121 angles) an iteration's data step and projection took 380 us as
+// transforms and element-wise passes of their own (copy of V, replacement, projection), and
+// takes 290 us (a third of it the projection's roots and divisions).
+struct LoadReal {
+    const float *p;
+    __device__ __forceinline__ float2 operator()(long i) const { return make_float2(__ldg(p + i), 0.f); }
+};
+
+constexpr int kTileVals = 512;   // packed values staged per tile
+
+template <class P>
+constexpr size_t data_z_smem()
 {
-    const float beta = (float)ctl->beta, keep = (float)(1.0 - ctl->beta);
-    const long i0 = (long)blockIdx.x * (kPer * kThreads) + threadIdx.x;
-    float2 f[kPer];
-#pragma unroll
-    for (int k = 0; k < kPer; k++) f[k] = i0 + k * kThreads < n ? F2[i0 + k * kThreads] : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < kPer; k++) {
-        if (f[k].x != 0.f || f[k].y != 0.f) {
-            const long i = i0 + k * kThreads;
-            const float2 g = G[i];
-            G[i] = make_float2(beta * (f[k].x * y_scale) + keep * g.x, beta * (f[k].y * y_scale) + keep * g.y);
-        }
-    }
+    return sizeof(float2) * (P::B * P::LP + kTileVals) + 2 * sizeof(int) * P::L;
 }
 
-__global__ void __launch_bounds__(kThreads) project_kernel(float2 *G, float *V, float *Vp, long n, float inv_n3,
-                                                           PocsCtl *ctl, double *part, bool write_g)
+// DD = false: F = beta Y + (1 - beta) F at the measured voxels, in place.  DD = true: only
+// the squared residual |F - Y|^2 over them, summed into ctl->dd.
+template <class P, bool DD>
+__global__ void __launch_bounds__(P::THREADS, P::E <= 16 ? 1024 / P::THREADS : 512 / P::THREADS)
+    data_z_kernel(LoopArgs a, float y_scale, PocsCtl *ctl, double *part, int ahead, const float2 *__restrict__ tw)
 {
+    constexpr int L = P::L;
+    extern __shared__ float4 smem4[];
+    float2 *buf = reinterpret_cast<float2 *>(smem4);
+    float2 *svals = buf + P::B * P::LP;
+    uint32_t *tm = reinterpret_cast<uint32_t *>(svals + kTileVals);
+    int *tp = reinterpret_cast<int *>(tm + L);
+    const long nl = (long)L * L;
+    const int nact = __ldg(a.zcount), id = blockIdx.x;
+    const bool live = id < nact;   // the same for the whole CTA
+    if (!DD && !live) return;
     float acc = 0.f;
-    for (long c = blockIdx.x; c * (kPer * kThreads) < n; c += gridDim.x) {
-        const long i0 = c * (kPer * kThreads) + threadIdx.x;
-        float2 g[kPer];
-        float v0[kPer];
-#pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            const long i = i0 + k * kThreads;
-            g[k] = i < n ? G[i] : make_float2(0.f, 0.f);
-            v0[k] = i < n ? V[i] : 0.f;
+    if (live) {
+        const long tile = __ldg(&a.ztiles[id]);
+        const int b = threadIdx.x % P::B, t = threadIdx.x / P::B;
+        float2 *line = a.G + tile * P::B + b;
+        const float2 *vals = a.tvals + tile * (long)P::B * L;
+        const int cnt = __ldg(&a.tcount[tile]);
+        if (ahead > 0 && id + ahead < nact) {
+            const float2 *nxt = a.G + (long)__ldg(&a.ztiles[id + ahead]) * P::B;
+            for (int z = threadIdx.x; z < L; z += P::THREADS) prefetch_l2(nxt + (long)z * nl);
         }
-#pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            const long i = i0 + k * kThreads;
-            if (i >= n) continue;
-            const float u = re_sqrt1p_m1(make_float2(g[k].x * inv_n3, g[k].y * inv_n3));
-            const float vn = u > 0.f ? u * (2.0f + u) : 0.f;
-            const float d = vn - v0[k];
-            acc = fmaf(d, d, acc);
-            V[i] = vn;
-            Vp[i] = vn;
-            if (write_g) G[i] = make_float2(vn, 0.f);
+        for (int z = threadIdx.x; z < L; z += P::THREADS) {
+            tm[z] = __ldg(&a.tmask[tile * L + z]);
+            tp[z] = __ldg(&a.tprefix[tile * L + z]);
         }
-    }
-    double t;
-    if (grid_sum(acc, part, &ctl->ticket, &t)) ctl->dp = sqrt(t);
-}
-
-__global__ void __launch_bounds__(kThreads) dd_kernel(const float2 *__restrict__ G, const float2 *__restrict__ F2,
-                                                      long n, float y_scale, PocsCtl *ctl, double *part)
-{
-    float acc = 0.f;
-    for (long c = blockIdx.x; c * (kPer * kThreads) < n; c += gridDim.x) {
-        const long i0 = c * (kPer * kThreads) + threadIdx.x;
-        float2 f[kPer];
+        for (int q = threadIdx.x; q < min(cnt, kTileVals); q += P::THREADS) svals[q] = __ldg(&vals[q]);
+        float2 v[P::E];
 #pragma unroll
-        for (int k = 0; k < kPer; k++) f[k] = i0 + k * kThreads < n ? F2[i0 + k * kThreads] : make_float2(0.f, 0.f);
+        for (int i = 0; i < P::E; i++) v[i] = __ldcs(&line[(long)fftl::slot_pos<L, P::T, P::F0>(i, t) * nl]);
+        const float beta = (float)ctl->beta, keep = (float)(1.0 - ctl->beta);
+        P::template seq<false, false, false>(buf, v, tw);   // its barriers also order the staging above
+        const uint32_t below = (1u << b) - 1u;
 #pragma unroll
-        for (int k = 0; k < kPer; k++) {
-            if (f[k].x != 0.f || f[k].y != 0.f) {
-                const float2 g = G[i0 + k * kThreads];
-                const float dx = g.x - f[k].x * y_scale, dy = g.y - f[k].y * y_scale;
-                acc = fmaf(dx, dx, fmaf(dy, dy, acc));
+        for (int i = 0; i < P::E; i++) {
+            const int z = fftl::slot_pos<L, P::T, P::RV0>(i, t);
+            const uint32_t m = tm[z];
+            if ((m >> b) & 1u) {
+                const int q = tp[z] + __popc(m & below);
+                const float2 f = q < kTileVals ? svals[q] : __ldg(&vals[q]);
+                if constexpr (DD) {
+                    const float dx = v[i].x - f.x * y_scale, dy = v[i].y - f.y * y_scale;
+                    acc = fmaf(dx, dx, fmaf(dy, dy, acc));
+                } else {
+                    v[i] = make_float2(beta * (f.x * y_scale) + keep * v[i].x, beta * (f.y * y_scale) + keep * v[i].y);
+                }
             }
         }
+        if constexpr (!DD) {
+            P::template seqr<true, false, false>(buf, v, tw);
+#pragma unroll
+            for (int i = 0; i < P::E; i++)
+                __stcs(&line[(long)fftl::slot_pos<L, P::T, P::F0>(i, t) * nl], cscale(v[i], a.inv_r));
+        }
     }
-    double t;
-    if (grid_sum(acc, part, &ctl->ticket, &t)) ctl->dd = sqrt(t);
+    if constexpr (DD) {
+        double tot;
+        if (grid_sum<P::THREADS>(acc, part, &ctl->ticket, &tot)) ctl->dd = sqrt(tot);
+    }
 }
+
+// IFFT_x of the rows and the projection V+ = (max(Re sqrt(1 + V), 1))^2 - 1 with Dp.
+template <class P>
+__global__ void __launch_bounds__(P::THREADS, row_min_ctas<P>())
+    rows_project_kernel(const float2 *__restrict__ G, float *V, float *Vp, float inv_r, PocsCtl *ctl, double *part,
+                        const float2 *__restrict__ tw)
+{
+    constexpr int L = P::L;   // the grid covers the L^2 rows exactly
+    extern __shared__ float4 smem4[];
+    const int t = threadIdx.x % P::T, b = threadIdx.x / P::T;
+    const long base = ((long)blockIdx.x * P::B + b) * L;
+    float2 v[P::E];
+    float v0[P::E];
+#pragma unroll
+    for (int i = 0; i < P::E; i++) v[i] = __ldcs(&G[base + fftl::slot_pos<L, P::T, P::F0>(i, t)]);
+#pragma unroll
+    for (int i = 0; i < P::E; i++) v0[i] = V[base + fftl::slot_pos<L, P::T, P::RV0>(i, t)];
+    P::template seq_row<true>(reinterpret_cast<float2 *>(smem4), v, tw);
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < P::E; i++) {
+        const long o = base + fftl::slot_pos<L, P::T, P::RV0>(i, t);
+        const float u = re_sqrt1p_m1(cscale(v[i], inv_r));
+        const float vn = u > 0.f ? u * (2.0f + u) : 0.f;
+        const float d = vn - v0[i];
+        acc = fmaf(d, d, acc);
+        V[o] = vn;
+        Vp[o] = vn;
+    }
+    double tot;
+    if (grid_sum<P::THREADS>(acc, part, &ctl->ticket, &tot)) ctl->dp = sqrt(tot);
+}
+
+// n = n_med sqrt(1 + V) (principal root, Re n >= n_med, Im n >= 0, as calculate_n3D),
+// octant shifted like cuFFT3Dshift.
+template <int L>
+struct StoreIndex {
+    float2 *ri;
+    float inv_r, n_med;
+    __device__ __forceinline__ void operator()(long i, float2 v) const
+    {
+        const unsigned u = (unsigned)i, x = u % L, yz = u / L, y = yz % L, z = yz / L, h = L / 2;   // L^3 < 2^31
+        ri[(x + h) % L + L * ((y + h) % L) + L * L * ((z + h) % L)] = est_n_scaled(v, inv_r, n_med);
+    }
+};
 
 // 1 / sqrt(x) by the hardware approximation (rsqrt.approx.ftz; x >= eps > 0 here, so
 // flushing subnormal inputs changes nothing).
@@ -181,137 +245,157 @@ __device__ __forceinline__ float rsqrt_approx(float x)
     return r;
 }
 
-// Gradient of TV at a voxel from the 13 values of its stencil (c: the voxel, xm / xp
-// the x neighbours, and so on; "xp_ym" the voxel at (+1, -1, 0)).  Each term is a
-// difference over the local gradient magnitude, taken with the reciprocal square root.
-__device__ __forceinline__ float tv_grad(float v, float vxm, float vym, float vzm, float vxp, float vyp, float vzp,
-                                         float xp_ym, float xp_zm, float xm_yp, float yp_zm, float xm_zp, float ym_zp,
-                                         float eps)
+// TV: a warp marches down through zc planes of one row of 32 VX voxels, VX consecutive
+// voxels per lane (16-byte loads at VX = 4).  A voxel's differences over its local magnitude,
+// q = (v - v_-d) / sqrt(eps + |..|^2), give the gradient as the sum of q over d at the voxel
+// minus q_d at its upper neighbours: x neighbours come by shuffle, z from the registers of
+// the march, and the warp computes the q_y of the row above itself (two magnitudes per voxel
+// where the 13-point stencil took four) from rows y - 1, y, y + 1, which its neighbours in
+// the CTA bring to L1 as well.  So no warp waits for another.  74.6 -> 58.0 us per step at
+// 256^3 (52 us for a streaming pass over the same 16 bytes a voxel).
+constexpr int kTy = 8;   // rows (warps) per CTA
+
+// Voxels per lane for side R, tiles (rows of a CTA) per plane.
+constexpr int tv_vx(int R) { return R % 128 == 0 ? 4 : R / 32; }
+int tv_tiles(int R) { return (R / (32 * tv_vx(R))) * (R / kTy); }
+// Planes per march (at least 4) that make the grid's waves shortest: waves of `resident`
+// CTAs, each one plane longer than its own planes.  256^3 on 456 resident CTAs: 7 chunks of
+// 37 planes, one wave; chunks of 32 took a second wave for the last 56 CTAs, and twice as long.
+int tv_planes(int R, int resident)
 {
-    const float a0 = v - vxm, b0 = v - vym, c0 = v - vzm;
-    const float r0 = rsqrt_approx(eps + a0 * a0 + b0 * b0 + c0 * c0);
-    const float ax = vxp - v, bx = vxp - xp_ym, cx = vxp - xp_zm;
-    const float rx = rsqrt_approx(eps + ax * ax + bx * bx + cx * cx);
-    const float ay = vyp - xm_yp, by = vyp - v, cy = vyp - yp_zm;
-    const float ry = rsqrt_approx(eps + ay * ay + by * by + cy * cy);
-    const float az = vzp - xm_zp, bz = vzp - ym_zp, cz = vzp - v;
-    const float rz = rsqrt_approx(eps + az * az + bz * bz + cz * cz);
-    return (a0 + b0 + c0) * r0 - ax * rx - by * ry - cz * rz;
-}
-
-// TV tile: 32 x 16 voxels of a plane per CTA (two rows per thread, eight apart),
-// marching through kZc planes along z with the planes z - 1, z, z + 1 (each with a
-// one-voxel periodic halo) in shared memory; the next plane's loads are issued before
-// the current plane is computed.  Every input element is read about 1.3 times.
-constexpr int kTx = 32, kTy = 16, kZc = 32;
-constexpr int kPw = kTx + 2, kPh = kTy + 2, kPlane = kPw * kPh, kLoads = (kPlane + kThreads - 1) / kThreads;
-
-int tv_blocks(int R) { return (R / kTx) * (R / kTy) * (R / kZc); }
-
-template <bool STEP>
-struct TvTile {
-    const float *__restrict__ Vin;
-    const float *__restrict__ gin;
-    float s;
-    int off[kLoads];    // plane offsets of this thread's tile elements (periodic halo)
-    int sidx[kLoads];   // their shared-memory index, -1 when unused
-
-    __device__ __forceinline__ void fetch(int base, float *r) const
-    {
-#pragma unroll
-        for (int j = 0; j < kLoads; j++) {
-            if (sidx[j] < 0) continue;
-            float v = __ldg(&Vin[base + off[j]]);
-            if constexpr (STEP) v = v - s * __ldg(&gin[base + off[j]]);
-            r[j] = v;
+    int best = R;
+    long cost = -1;
+    for (int zc = 4; zc <= R; zc++) {
+        const long ctas = (long)tv_tiles(R) * ((R + zc - 1) / zc);
+        const long c = (resident > 0 ? (ctas + resident - 1) / resident : ctas) * (zc + 1);
+        if (cost < 0 || c < cost) {
+            cost = c;
+            best = zc;
         }
     }
-    __device__ __forceinline__ void put(float *plane, const float *r) const
-    {
-#pragma unroll
-        for (int j = 0; j < kLoads; j++)
-            if (sidx[j] >= 0) plane[sidx[j]] = r[j];
-    }
-};
+    return best;
+}
 
-// The two voxels of this thread on plane pc (rows ly and ly + 8).
-__device__ __forceinline__ void tv_two(const float (*pm)[kPw], const float (*pc)[kPw], const float (*pp)[kPw], int lx,
-                                       int ly, float eps, float *v, float *g)
+template <int VX>
+__device__ __forceinline__ void ld_vec(const float *__restrict__ p, float *v)
 {
+    if constexpr (VX == 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
+        v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+    } else {
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const int y = ly + 8 * h;
-        v[h] = pc[y][lx];
-        g[h] = tv_grad(v[h], pc[y][lx - 1], pc[y - 1][lx], pm[y][lx], pc[y][lx + 1], pc[y + 1][lx], pp[y][lx],
-                       pc[y - 1][lx + 1], pm[y][lx + 1], pc[y + 1][lx - 1], pm[y + 1][lx], pp[y][lx - 1],
-                       pp[y - 1][lx], eps);
+        for (int k = 0; k < VX; k++) v[k] = __ldg(p + k);
+    }
+}
+template <int VX>
+__device__ __forceinline__ void st_vec(float *p, const float *v)
+{
+    if constexpr (VX == 4) {
+        *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < VX; k++) p[k] = v[k];
     }
 }
 
-// STEP = false: g = grad TV(Vin).  STEP = true: the volume is Vin - s gin with
+// Rows y - 1, y, y + 1 of a plane: VX voxels per lane, and for lane 0 / 31 the voxel left /
+// right of the row segment.
+template <int VX>
+struct TvRows {
+    float v[3][VX], h[3];
+};
+
+// STEP = false: gout = grad TV(Vin).  STEP = true: the volume is Vin - s gin with
 // s = dtvg / |gin| (the previous descent step, applied while the planes are loaded),
 // written to Vout, and gout = grad TV of it.  The last block stores |gout| and, on the
 // first iteration, sets dtvg = alpha Dp.  Offsets are 32-bit (R^3 < 2^31 for R <= 768).
-template <bool STEP>
-__global__ void __launch_bounds__(kThreads) tv_kernel(const float *__restrict__ Vin, const float *__restrict__ gin,
-                                                      float *Vout, float *gout, int R, float eps, PocsCtl *ctl,
-                                                      double *part)
+template <bool STEP, int VX>
+__global__ void __launch_bounds__(kThreads, 3) tv_kernel(const float *__restrict__ Vin, const float *__restrict__ gin,
+                                                         float *Vout, float *gout, int R, int zc, float eps,
+                                                         PocsCtl *ctl, double *part)
 {
-    static_assert(kTx * kTy == 2 * kThreads, "two voxels of the tile per thread");
-    __shared__ float pl[3][kPh][kPw];
-    TvTile<STEP> t;
-    t.Vin = Vin;
-    t.gin = gin;
-    t.s = 0.f;
-    if constexpr (STEP) t.s = ctl->gnorm > 0.0 ? (float)(ctl->dtvg / ctl->gnorm) : 0.f;
-    const int nbx = R / kTx, nby = R / kTy;
+    static_assert(kThreads == 32 * kTy, "a warp per row");
+    constexpr int TX = 32 * VX;
+    float step = 0.f;
+    if constexpr (STEP) step = ctl->gnorm > 0.0 ? (float)(ctl->dtvg / ctl->gnorm) : 0.f;
+    const int lane = threadIdx.x & 31;
+    const int nbx = R / TX, nby = R / kTy;
     int bi = blockIdx.x;
-    const int x0 = (bi % nbx) * kTx;
+    const int x0 = (bi % nbx) * TX;
     bi /= nbx;
-    const int y0 = (bi % nby) * kTy, z0 = (bi / nby) * kZc;
-    const int rr = R * R;
+    const int y = (bi % nby) * kTy + (threadIdx.x >> 5), z0 = (bi / nby) * zc, z1 = min(z0 + zc, R);
+    const int rr = R * R, x = x0 + lane * VX;
+    const int row[3] = {R * (y == 0 ? R - 1 : y - 1), R * y, R * (y + 1 == R ? 0 : y + 1)};
+    const bool edge = lane == 0 || lane == 31;
+    const int xh = lane == 0 ? (x0 == 0 ? R - 1 : x0 - 1) : (x0 + TX == R ? 0 : x0 + TX);
+    using Rows = TvRows<VX>;
+    auto fetch = [&](int z, Rows &a, Rows &b) {
+        const int base = rr * (z < 0 ? z + R : (z >= R ? z - R : z));
 #pragma unroll
-    for (int j = 0; j < kLoads; j++) {
-        const int e = threadIdx.x + j * kThreads;
-        const int lx = e % kPw, ly = e / kPw;
-        int gx = x0 - 1 + lx, gy = y0 - 1 + ly;
-        gx = gx < 0 ? gx + R : (gx >= R ? gx - R : gx);
-        gy = gy < 0 ? gy + R : (gy >= R ? gy - R : gy);
-        t.sidx[j] = e < kPlane ? e : -1;
-        t.off[j] = e < kPlane ? gx + R * gy : 0;
-    }
-    auto zbase = [&](int z) { return rr * (z < 0 ? z + R : (z >= R ? z - R : z)); };
-    const int tx = threadIdx.x % kTx, ty = threadIdx.x / kTx, lx = tx + 1, ly = ty + 1;
-    const int out0 = (x0 + tx) + R * (y0 + ty);
-    float nxt[kLoads];
-    t.fetch(zbase(z0 - 1), nxt);
-    t.put(&pl[0][0][0], nxt);
-    t.fetch(zbase(z0), nxt);
-    t.put(&pl[1][0][0], nxt);
-    t.fetch(zbase(z0 + 1), nxt);
-    float acc = 0.f;
-    auto plane_step = [&](int k, float *pnew, const float (*pm)[kPw], const float (*pc)[kPw],
-                          const float (*pp)[kPw]) {
-        t.put(pnew, nxt);   // plane z0 + k + 1
-        __syncthreads();
-        if (k + 1 < kZc) t.fetch(zbase(z0 + k + 2), nxt);   // in flight while this plane is computed
-        float v[2], g[2];
-        tv_two(pm, pc, pp, lx, ly, eps, v, g);
-        const int q = out0 + rr * (z0 + k);
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            if constexpr (STEP) Vout[q + 8 * R * h] = v[h];
-            gout[q + 8 * R * h] = g[h];
-            acc = fmaf(g[h], g[h], acc);
+        for (int d = 0; d < 3; d++) {
+            ld_vec<VX>(Vin + base + row[d] + x, a.v[d]);
+            a.h[d] = edge ? __ldg(&Vin[base + row[d] + xh]) : 0.f;
+            if constexpr (STEP) {
+                ld_vec<VX>(gin + base + row[d] + x, b.v[d]);
+                b.h[d] = edge ? __ldg(&gin[base + row[d] + xh]) : 0.f;
+            }
         }
-        __syncthreads();
     };
-    for (int k = 0; k < kZc; k++) {
-        switch (k % 3) {   // plane slots as constants: z - 1, z, z + 1
-        case 0: plane_step(k, &pl[2][0][0], pl[0], pl[1], pl[2]); break;
-        case 1: plane_step(k, &pl[0][0][0], pl[1], pl[2], pl[0]); break;
-        default: plane_step(k, &pl[1][0][0], pl[2], pl[0], pl[1]); break;
+    auto take = [&](const Rows &a, const Rows &b, Rows &o) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+#pragma unroll
+            for (int k = 0; k < VX; k++) o.v[d][k] = STEP ? a.v[d][k] - step * b.v[d][k] : a.v[d][k];
+            o.h[d] = STEP ? a.h[d] - step * b.h[d] : a.h[d];
         }
+    };
+    Rows la, lb, c, m;   // loads in flight; planes z and z - 1
+    float qz[VX];        // q_z one plane above
+    fetch(z1, la, lb);
+    take(la, lb, c);
+    fetch(z1 - 1, la, lb);
+    float acc = 0.f;
+    // plane z1 only gives q_z
+    for (int z = z1; z >= z0; z--) {
+        take(la, lb, m);
+        if (z > z0) fetch(z - 2, la, lb);   // in flight while this plane is computed
+        float left[2];                      // x - 1 of the lane's first voxel, rows y and y + 1
+#pragma unroll
+        for (int d = 0; d < 2; d++) {
+            const float up = __shfl_up_sync(0xffffffffu, c.v[d + 1][VX - 1], 1);
+            left[d] = lane == 0 ? c.h[d + 1] : up;
+        }
+        float s[VX], qx[VX], qzn[VX], qyu[VX];
+#pragma unroll
+        for (int k = 0; k < VX; k++) {
+            const float p = c.v[1][k], u = c.v[2][k];
+            const float da = p - (k ? c.v[1][k - 1] : left[0]), db = p - c.v[0][k], dc = p - m.v[1][k];
+            const float r = rsqrt_approx(eps + da * da + db * db + dc * dc);
+            s[k] = (da + db + dc) * r;
+            qx[k] = da * r;
+            qzn[k] = dc * r;
+            const float ua = u - (k ? c.v[2][k - 1] : left[1]), ub = u - p, uc = u - m.v[2][k];
+            qyu[k] = ub * rsqrt_approx(eps + ua * ua + ub * ub + uc * uc);
+        }
+        float qr = __shfl_down_sync(0xffffffffu, qx[0], 1);
+        if (lane == 31) {
+            const float da = c.h[1] - c.v[1][VX - 1], db = c.h[1] - c.h[0], dc = c.h[1] - m.h[1];
+            qr = da * rsqrt_approx(eps + da * da + db * db + dc * dc);
+        }
+        if (z < z1) {
+            float g[VX];
+#pragma unroll
+            for (int k = 0; k < VX; k++) {
+                g[k] = s[k] - qz[k] - (k + 1 < VX ? qx[k + 1 < VX ? k + 1 : 0] : qr) - qyu[k];
+                acc = fmaf(g[k], g[k], acc);
+            }
+            const int o = x + row[1] + rr * z;
+            if constexpr (STEP) st_vec<VX>(Vout + o, c.v[1]);
+            st_vec<VX>(gout + o, g);
+        }
+#pragma unroll
+        for (int k = 0; k < VX; k++) qz[k] = qzn[k];
+        c = m;
     }
     double tot;
     if (grid_sum(acc, part, &ctl->ticket, &tot)) {
@@ -323,11 +407,20 @@ __global__ void __launch_bounds__(kThreads) tv_kernel(const float *__restrict__ 
     }
 }
 
-// The last descent step, Dg, the step-size rule and the history entry; G = V for the
-// next iteration's transform.
+template <bool STEP>
+cudaError_t launch_tv(const float *Vin, const float *gin, float *Vout, float *gout, const PocsBufs &b, cudaStream_t s)
+{
+    auto k = tv_vx(b.R) == 4 ? tv_kernel<STEP, 4> : (tv_vx(b.R) == 2 ? tv_kernel<STEP, 2> : tv_kernel<STEP, 1>);
+    const int zc = tv_planes(b.R, wave_ctas(k, kThreads, 0));
+    k<<<(unsigned)(tv_tiles(b.R) * ((b.R + zc - 1) / zc)), kThreads, 0, s>>>(Vin, gin, Vout, gout, b.R, zc, b.tv_eps,
+                                                                            b.ctl, b.part);
+    note_launch();
+    return cudaGetLastError();
+}
+
+// The last descent step, Dg, the step-size rule and the history entry.
 __global__ void __launch_bounds__(kThreads) tv_final_kernel(const float *Vin, const float *gin, float *V,
-                                                            const float *__restrict__ Vp, float2 *G, long n,
-                                                            PocsCtl *ctl, double *part, double *hist)
+                                                            const float *__restrict__ Vp, long n, PocsCtl *ctl, double *part, double *hist)
 {
     const float s = ctl->gnorm > 0.0 ? (float)(ctl->dtvg / ctl->gnorm) : 0.f;
     float acc = 0.f;
@@ -349,7 +442,6 @@ __global__ void __launch_bounds__(kThreads) tv_final_kernel(const float *Vin, co
             const float d = v - pi[k];
             acc = fmaf(d, d, acc);
             V[i] = v;
-            G[i] = make_float2(v, 0.f);
         }
     }
     double t;
@@ -368,28 +460,6 @@ __global__ void __launch_bounds__(kThreads) tv_final_kernel(const float *Vin, co
     }
 }
 
-// n = n_med sqrt(1 + V) (principal root, Re n >= n_med, Im n >= 0, as calculate_n3D),
-// octant shifted like cuFFT3Dshift.
-__global__ void __launch_bounds__(kThreads) pocs_n_kernel(const float2 *__restrict__ G, int R, float inv_n3,
-                                                          float n_med, float2 *ri)
-{
-    // 32-bit index arithmetic: R^3 < 2^31 for R <= 768
-    const unsigned ur = (unsigned)R, rr = ur * ur, n = rr * ur, h = ur / 2;
-    const unsigned i0 = blockIdx.x * (kPer * kThreads) + threadIdx.x;
-    float2 g[kPer];
-#pragma unroll
-    for (int k = 0; k < kPer; k++) g[k] = i0 + k * kThreads < n ? G[i0 + k * kThreads] : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < kPer; k++) {
-        const unsigned i = i0 + k * kThreads;
-        if (i >= n) continue;
-        const unsigned x = i % ur, yz = i / ur, y = yz % ur, z = yz / ur;
-        const unsigned xs = x + h >= ur ? x + h - ur : x + h, ys = y + h >= ur ? y + h - ur : y + h,
-                       zs = z + h >= ur ? z + h - ur : z + h;
-        ri[xs + ur * ys + rr * zs] = est_n_scaled(g[k], inv_n3, n_med);
-    }
-}
-
 unsigned grid_for(long n) { return (unsigned)((n + kPer * kThreads - 1) / (kPer * kThreads)); }
 
 // Reducing elementwise kernels: at most 8 CTAs per SM of 152, each looping over chunks
@@ -401,80 +471,137 @@ unsigned grid_reduce(long n)
     return g < kReduceGrid ? g : kReduceGrid;
 }
 
-cudaError_t fft3_unscaled(float2 *G, int R, bool inverse, cudaStream_t s)
-{
-    const long rr = (long)R * R;
-    cudaError_t e = fft_rows(G, R, rr, inverse, s);
-    if (e == cudaSuccess) e = fft_cols(G, R, rr, R, rr, R, inverse, s);
-    if (e == cudaSuccess) e = fft_cols(G, R, rr, R, R, rr, inverse, s);
-    return e;
-}
+// Launchers per volume side.
+template <int L>
+struct Lines {
+    using P = TilePlan<L>;
+    static LoopArgs args(const PocsBufs &b)
+    {
+        LoopArgs a = {};
+        a.G = b.G;
+        a.inv_r = 1.0f / (float)L;
+        a.tmask = b.tmask;
+        a.tcount = b.tcount;
+        a.tprefix = b.tprefix;
+        a.tvals = b.tvals;
+        active_view(a, b.active, L);
+        return a;
+    }
+    template <bool DD>
+    static cudaError_t z(const PocsBufs &b, cudaStream_t s)
+    {
+        const size_t smem = data_z_smem<P>();
+        auto k = data_z_kernel<P, DD>;
+        const cudaError_t e = prep_line_kernel(reinterpret_cast<const void *>(k), L, smem);
+        if (e != cudaSuccess) return e;
+        k<<<(unsigned)((long)L * L / P::B), P::THREADS, smem, s>>>(args(b), b.y_scale, b.ctl, b.part,
+                                                                  wave_ctas(k, P::THREADS, smem), twiddles(L));
+        note_launch();
+        return cudaGetLastError();
+    }
+    static cudaError_t y(const PocsBufs &b, bool inverse, cudaStream_t s)
+    {
+        const long rr = (long)L * L;
+        return fft_cols_from(b.G, b.G, L, rr, L, rr, L, inverse, inverse ? 1.0f / (float)L : 1.0f, s, b.active + 4);
+    }
+    // V's spectrum up to the z lines
+    static cudaError_t forward(const PocsBufs &b, cudaStream_t s)
+    {
+        const cudaError_t e = rows_fn_launch<RowPlan<L>, false>(LoadReal{b.V}, StoreScaled{b.G, 1.0f}, (long)L * L, s);
+        return e == cudaSuccess ? y(b, false, s) : e;
+    }
+    // FFT3(V) -> data step -> IFFT_z, IFFT_y (normalised; IFFT_x and its 1 / R follow)
+    static cudaError_t data(const PocsBufs &b, cudaStream_t s)
+    {
+        cudaError_t e = forward(b, s);
+        if (e == cudaSuccess) e = z<false>(b, s);
+        return e == cudaSuccess ? y(b, true, s) : e;
+    }
+    static cudaError_t project(const PocsBufs &b, cudaStream_t s)
+    {
+        using PR = RowPlan<L>;
+        cudaError_t e = data(b, s);
+        if (e != cudaSuccess) return e;
+        const size_t smem = fftl::plan_smem_row<PR>();
+        auto k = rows_project_kernel<PR>;
+        if ((e = prep_line_kernel(reinterpret_cast<const void *>(k), L, smem)) != cudaSuccess) return e;
+        k<<<(unsigned)((long)L * L / PR::B), PR::THREADS, smem, s>>>(b.G, b.V, b.Vp, 1.0f / (float)L, b.ctl, b.part,
+                                                                    twiddles(L));
+        note_launch();
+        return cudaGetLastError();
+    }
+    static cudaError_t residual(const PocsBufs &b, cudaStream_t s)
+    {
+        const cudaError_t e = forward(b, s);
+        return e == cudaSuccess ? z<true>(b, s) : e;
+    }
+    static cudaError_t finish(const PocsBufs &b, float n_med, float2 *ri, cudaStream_t s)
+    {
+        const cudaError_t e = data(b, s);
+        if (e != cudaSuccess) return e;
+        return rows_fn_launch<RowPlan<L>, true>(LoadComplex{b.G}, StoreIndex<L>{ri, 1.0f / (float)L, n_med},
+                                                (long)L * L, s);
+    }
+};
 
-// FFT3(G) -> data step -> IFFT3 (unscaled; the 1/R^3 is applied by the consumer).
-cudaError_t data_step(const PocsBufs &b, cudaStream_t s)
+#define CTDM_LINES(R, CALL)                                  \
+    switch (R) {                                             \
+    case 32: return Lines<32>::CALL;                         \
+    case 64: return Lines<64>::CALL;                         \
+    case 128: return Lines<128>::CALL;                       \
+    case 256: return Lines<256>::CALL;                       \
+    case 384: return Lines<384>::CALL;                       \
+    case 512: return Lines<512>::CALL;                       \
+    case 768: return Lines<768>::CALL;                       \
+    default: return cudaErrorInvalidValue;                   \
+    }
+cudaError_t project_lines(const PocsBufs &b, cudaStream_t s) { CTDM_LINES(b.R, project(b, s)) }
+cudaError_t residual_lines(const PocsBufs &b, cudaStream_t s) { CTDM_LINES(b.R, residual(b, s)) }
+cudaError_t finish_lines(const PocsBufs &b, float n_med, float2 *ri, cudaStream_t s)
 {
-    const long n = (long)b.R * b.R * b.R;
-    cudaError_t e = fft3_unscaled(b.G, b.R, false, s);
-    if (e != cudaSuccess) return e;
-    dc_kernel<<<grid_for(n), kThreads, 0, s>>>(b.G, b.F2, n, b.ctl, b.y_scale);
-    note_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return fft3_unscaled(b.G, b.R, true, s);
+    CTDM_LINES(b.R, finish(b, n_med, ri, s))
 }
 
 }  // namespace
 
 int pocs_partials(int R)
 {
-    const int t = tv_blocks(R), e = (int)grid_for((long)R * R * R);
-    return t > e ? t : e;
+    // tiles of at least 8 lines, rows of at least 8 per CTA, TV blocks, reducing passes
+    const long t = (long)tv_tiles(R) * ((R + 3) / 4), l = (long)R * R / 8, e = kReduceGrid;
+    return (int)(t > l ? (t > e ? t : e) : (l > e ? l : e));
 }
+
+int pocs_tile(int R) { return tile_lines(R); }
 
 cudaError_t pocs_iteration(const PocsBufs &b, int tv_steps, bool want_dd, cudaStream_t s)
 {
     const int R = b.R;
     const long n = (long)R * R * R;
-    const float inv_n3 = 1.0f / (float)n;
-    cudaError_t e = data_step(b, s);
+    cudaError_t e = project_lines(b, s);
+    if (e == cudaSuccess && want_dd) e = residual_lines(b, s);
     if (e != cudaSuccess) return e;
-    project_kernel<<<grid_reduce(n), kThreads, 0, s>>>(b.G, b.V, b.Vp, n, inv_n3, b.ctl, b.part, want_dd);
-    note_launch();
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if (want_dd) {
-        if ((e = fft3_unscaled(b.G, R, false, s)) != cudaSuccess) return e;
-        dd_kernel<<<grid_reduce(n), kThreads, 0, s>>>(b.G, b.F2, n, b.y_scale, b.ctl, b.part);
-        note_launch();
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
     // TV steepest descent: gradient at the POCS result, then tv_steps - 1 fused
     // (step, gradient) passes between two buffer pairs, then the last step
-    const unsigned tvg = (unsigned)tv_blocks(R);
-    tv_kernel<false><<<tvg, kThreads, 0, s>>>(b.V, nullptr, nullptr, b.g, R, b.tv_eps, b.ctl, b.part);
-    note_launch();
+    e = launch_tv<false>(b.V, nullptr, nullptr, b.g, b, s);
     const float *vin = b.V, *gin = b.g;
     float *vout = b.V2, *gout = b.g2;
-    for (int t = 1; t < tv_steps; t++) {
-        tv_kernel<true><<<tvg, kThreads, 0, s>>>(vin, gin, vout, gout, R, b.tv_eps, b.ctl, b.part);
-        note_launch();
+    for (int t = 1; t < tv_steps && e == cudaSuccess; t++) {
+        e = launch_tv<true>(vin, gin, vout, gout, b, s);
         const float *nv = vout, *ng = gout;
         vout = const_cast<float *>(vin);
         gout = const_cast<float *>(gin);
         vin = nv;
         gin = ng;
     }
-    tv_final_kernel<<<grid_reduce(n), kThreads, 0, s>>>(vin, gin, b.V, b.Vp, b.G, n, b.ctl, b.part, b.hist);
+    if (e != cudaSuccess) return e;
+    tv_final_kernel<<<grid_reduce(n), kThreads, 0, s>>>(vin, gin, b.V, b.Vp, n, b.ctl, b.part, b.hist);
     note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t pocs_finish(const PocsBufs &b, float n_med, float2 *ri, cudaStream_t s)
 {
-    const long n = (long)b.R * b.R * b.R;
-    cudaError_t e = data_step(b, s);
-    if (e != cudaSuccess) return e;
-    pocs_n_kernel<<<grid_for(n), kThreads, 0, s>>>(b.G, b.R, 1.0f / (float)n, n_med, ri);
-    note_launch();
-    return cudaGetLastError();
+    return finish_lines(b, n_med, ri, s);
 }
 
 }  // namespace ctdm

@@ -431,7 +431,8 @@ static cudaError_t ewald_launch(const EwaldArgs &a, cudaStream_t s)
 template <int TB>
 __global__ void __launch_bounds__(256) pack_measured_kernel(const float2 *__restrict__ F2,
                                                            const uint8_t *__restrict__ mask, int R, uint32_t *tmask,
-                                                           int *tcount, int *tprefix, float2 *tvals, int *active)
+                                                           int *tcount, int *tprefix, float2 *tvals, int *active,
+                                                           PackRule rule)
 {
     extern __shared__ int spre[];   // R prefixes, then 8 warp totals
     int *swarp = spre + R;
@@ -452,7 +453,7 @@ __global__ void __launch_bounds__(256) pack_measured_kernel(const float2 *__rest
                 keep = mask[idx] != 0;
             } else {
                 const float2 f = F2[idx];
-                keep = f.x != 0.0f && f.y != 0.0f;
+                keep = rule == PACK_BOTH ? f.x != 0.0f && f.y != 0.0f : f.x != 0.0f || f.y != 0.0f;
             }
         }
         const unsigned bal = __ballot_sync(0xffffffffu, keep);
@@ -513,15 +514,15 @@ __global__ void __launch_bounds__(256) pack_measured_kernel(const float2 *__rest
 }
 
 cudaError_t pack_measured(const float2 *F2, const uint8_t *mask, int R, int TB, uint32_t *tmask, int *tcount,
-                          int *tprefix, float2 *tvals, int *active, cudaStream_t s)
+                          int *tprefix, float2 *tvals, int *active, cudaStream_t s, PackRule rule)
 {
     if (R > 768) return cudaErrorInvalidValue;
     const unsigned tiles = (unsigned)((long)R * R / TB);
     const size_t smem = sizeof(int) * (R + 8);
     switch (TB) {
-    case 8: pack_measured_kernel<8><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active); break;
-    case 16: pack_measured_kernel<16><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active); break;
-    case 32: pack_measured_kernel<32><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active); break;
+    case 8: pack_measured_kernel<8><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active, rule); break;
+    case 16: pack_measured_kernel<16><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active, rule); break;
+    case 32: pack_measured_kernel<32><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active, rule); break;
     default: return cudaErrorInvalidValue;
     }
     note_launch();

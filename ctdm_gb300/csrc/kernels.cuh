@@ -54,8 +54,11 @@ struct LoopArgs {
     float2 *out;            // final RI volume (octant shifted), only for the final pass
     int R;
     float k2, n_med, n_med2;
-    float s1;   // -1 / (R^2 k^2) on the plane scheme, -1 / (R k^2) on the line passes
-    float inv_r;   // 1 / R: the z passes (and the y inverse pass) leave normalised lines
+    // -1 / (S k^2) with S what the inverse transforms leave unnormalised: R^3, or where
+    // empty tiles are skipped R^2 on the plane scheme and R on the line passes
+    float s1;
+    float inv_r;   // 1 / R: where empty tiles are skipped the z passes (and the y inverse
+                   // pass) leave normalised lines
     float s2;   // -k^2 / n_med^2
     int *err;   // device status word: a bounded wait that ran out records a nonzero code
     int staged; // z pass: F2 / mask tiles staged by TMA (set by the launcher)
@@ -78,7 +81,12 @@ struct LoopArgs {
     float beta;
 };
 
-// Packs F2 (mode 0: re != 0 && im != 0; mode 1: mask != 0) into per-tile masks,
+// Whether the loop of side R leaves out what no measured voxel touches (loop_passes.cuh).
+__host__ __device__ constexpr bool skip_empty_tiles(int R) { return R > 128; }
+// Which voxels of F2 pack_measured keeps without a mask: both parts non-zero (the loop's
+// reference predicate) or any part (POCS).
+enum PackRule { PACK_BOTH, PACK_NONZERO };
+// Packs F2 (the rule's voxels, or with a mask those where it is non-zero) into per-tile masks,
 // counts, row prefixes and values for the z pass (TB lines per tile, 8, 16 or 32), and
 // lists the tiles that keep a sample: active holds a header {count, 3 unused, R / 8
 // column flags}, zero before the call, and the tile list (active_ints(R) entries, enough
@@ -86,7 +94,7 @@ struct LoopArgs {
 // passes take every tile (skip_empty_tiles, loop_passes.cuh), tvals where the values are
 // kept elsewhere.
 cudaError_t pack_measured(const float2 *F2, const uint8_t *mask, int R, int TB, uint32_t *tmask, int *tcount,
-                          int *tprefix, float2 *tvals, int *active, cudaStream_t s);
+                          int *tprefix, float2 *tvals, int *active, cudaStream_t s, PackRule rule = PACK_BOTH);
 __host__ __device__ inline int active_head(int R) { return 4 + R / 8; }
 inline size_t active_ints(int R) { return active_head(R) + (size_t)R * R / 8; }
 inline void active_view(LoopArgs &a, const int *active, int R)
@@ -152,7 +160,10 @@ struct PocsCtl {
 struct PocsBufs {
     float *V, *g, *V2, *g2, *Vp;   // real R^3 volumes (contrast, TV gradient, ping-pong, POCS result)
     float2 *G;                     // complex R^3 work volume
-    const float2 *F2;              // measured k-space data (zero where nothing was measured)
+    // measured k-space data by z tile (pack_measured, PACK_NONZERO, tiles of pocs_tile(R) lines)
+    const uint32_t *tmask;
+    const int *tcount, *tprefix, *active;
+    const float2 *tvals;
     double *part;                  // per-block partial sums (pocs_partials(R))
     PocsCtl *ctl;
     double *hist;                  // 4 doubles per iteration: Dp, Dd, Dg, the TV step used
@@ -162,6 +173,8 @@ struct PocsBufs {
 };
 // Partial-sum slots a run of side R needs.
 int pocs_partials(int R);
+// Lines per z tile of the packed samples.
+int pocs_tile(int R);
 cudaError_t pocs_iteration(const PocsBufs &b, int tv_steps, bool want_dd, cudaStream_t s);
 // After the last iteration: one more data-consistency step, then n = n_med sqrt(1 + V)
 // with Re n >= n_med, Im n >= 0, octant shifted into ri.

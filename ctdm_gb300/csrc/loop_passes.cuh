@@ -135,13 +135,6 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4)) xpass_k
     }
 }
 
-// Whether the passes of side L leave out what no measured voxel touches (see the z pass).
-template <int L>
-constexpr bool skip_empty_tiles()
-{
-    return L > 128;
-}
-
 // ------------------------------------------------------------ y pass
 // Lines (x, z) with B consecutive x per CTA (coalesced B*8-byte segments per row).
 // Columns x over which no voxel is measured (xactive) pass through the z pass unchanged,
@@ -160,7 +153,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(5)) ypass_k
     const int b = threadIdx.x % P::B, t = threadIdx.x / P::B;
     const long l = line0 + b;
     const long base = (l % L) + (l / L) * (long)L * L;
-    if (skip_empty_tiles<L>() && a.xactive) {
+    if (skip_empty_tiles(L) && a.xactive) {
         int any = 0;   // the same for every thread: a CTA's B columns share one z
         const int x0 = (int)(line0 % L);
 #pragma unroll
@@ -173,7 +166,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(5)) ypass_k
     P::template seq<INV, false, false>(buf, v, tw);
 #pragma unroll
     for (int i = 0; i < P::E; i++)
-        __stcs(&a.G[base + (long)fftl::slot_pos<L, P::T, P::RV0>(i, t) * L], INV ? cscale(v[i], a.inv_r) : v[i]);
+        __stcs(&a.G[base + (long)fftl::slot_pos<L, P::T, P::RV0>(i, t) * L], INV && skip_empty_tiles(L) ? cscale(v[i], a.inv_r) : v[i]);
 }
 
 // ------------------------------------------------------------ z pass
@@ -259,7 +252,8 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(3))
     P::template seqr<true, false, false>(buf, v, tw);
 #pragma unroll
     for (int i = 0; i < P::E; i++)
-        __stcs(&a.G[base + (long)fftl::slot_pos<L, P::T, P::F0>(i, t) * nl], cscale(v[i], a.inv_r));
+        __stcs(&a.G[base + (long)fftl::slot_pos<L, P::T, P::F0>(i, t) * nl],
+               skip_empty_tiles(L) ? cscale(v[i], a.inv_r) : v[i]);
 }
 
 // ------------------------------------------------------------ z pass on packed measured samples
@@ -276,7 +270,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(3))
 // lateral frequencies up to (n + NA) / lambda), and the pass went from 58.7 to 41.2 us
 // per launch at 256^3.  Volumes up to 128^3 run in about one wave, where the list's
 // extra load costs more than the skipped tiles give (3.9 -> 4.3 us per launch at 64^3):
-// they take every tile in order.
+// they take every tile in order and leave their lines unnormalised.
 constexpr int ZCAP = 1024;
 
 template <class P>
@@ -307,7 +301,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4))
     float2 *buf = reinterpret_cast<float2 *>(spre + L + 16);
     uint64_t *bar = reinterpret_cast<uint64_t *>(buf + P::B * P::LP);
     const long nl = (long)L * L;
-    constexpr bool SKIP = skip_empty_tiles<L>();
+    constexpr bool SKIP = skip_empty_tiles(L);
     const int nact = SKIP ? __ldg(a.zcount) : (int)gridDim.x;
     if ((int)blockIdx.x >= nact) return;
     const long tile = SKIP ? __ldg(&a.ztiles[blockIdx.x]) : (long)blockIdx.x;
@@ -347,7 +341,8 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4))
     P::template seqr<true, false, false>(buf, v, tw);
 #pragma unroll
     for (int i = 0; i < P::E; i++)
-        __stcs(&a.G[base + (long)fftl::slot_pos<L, P::T, P::F0>(i, t) * nl], cscale(v[i], a.inv_r));
+        __stcs(&a.G[base + (long)fftl::slot_pos<L, P::T, P::F0>(i, t) * nl],
+               skip_empty_tiles(L) ? cscale(v[i], a.inv_r) : v[i]);
 }
 
 // ------------------------------------------------------------ launchers
