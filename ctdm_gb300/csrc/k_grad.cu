@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kTvThreads, 3) tv_kernel(TvArgs a)
     int bi = blockIdx.x;
     const int x0 = (bi % nbx) * kTvX;
     bi /= nbx;
-    const int y0 = (bi % nby) * kTvY, z0 = (bi / nby) * a.zc;
+    const int y0 = (bi % nby) * kTvY, z0 = (bi / nby) * a.zc, z1 = min(z0 + a.zc, R);
     const int rr = R * R;   // R^3 < 2^31 for R <= 768
     int off[kTvLoads];
 #pragma unroll
@@ -455,10 +455,10 @@ __global__ void __launch_bounds__(kTvThreads, 3) tv_kernel(TvArgs a)
     put(&pl[(z0 - 1) & 1][0][0], nxt);
     fetch(z0, nxt);
     // plane z0 - 1 only gives q_z (nothing below the volume)
-    for (int z = z0 - 1; z < z0 + a.zc; z++) {
+    for (int z = z0 - 1; z < z1; z++) {
         put(&pl[(z + 1) & 1][0][0], nxt);
         __syncthreads();
-        if (z + 1 < z0 + a.zc) fetch(z + 2, nxt);
+        if (z + 1 < z1) fetch(z + 2, nxt);
         const float2(*pc)[kTvW] = pl[z & 1], (*pn)[kTvW] = pl[(z + 1) & 1];
         float2 div[2], c[2], gv[2], vv[2];
         const bool own = z >= z0;
@@ -526,21 +526,25 @@ __global__ void __launch_bounds__(kTvThreads, 3) tv_kernel(TvArgs a)
     if (a.partial) block_partial(acc, a.partial);
 }
 
-// Planes per CTA of the TV march: 32, fewer on small volumes so that the grid holds at
-// least two CTAs per SM where the volume allows (each march starts with two extra planes).
+int tv_tiles(int R) { return (R / kTvX) * (R / kTvY); }
+// Planes per CTA of the march and CTAs of the grid.
+template <bool UPDATE>
 int tv_planes(int R)
 {
-    int zc = 32;
-    while (zc > 4 && (long)(R / kTvX) * (R / kTvY) * (R / zc) < 304) zc /= 2;
-    return zc;
+    return march_planes(R, tv_tiles(R), wave_ctas(tv_kernel<UPDATE>, kTvThreads, 0));
 }
-unsigned tv_grid(int R) { return (unsigned)((R / kTvX) * (R / kTvY) * (R / tv_planes(R))); }
+template <bool UPDATE>
+unsigned tv_grid(int R)
+{
+    const int zc = tv_planes<UPDATE>(R);
+    return (unsigned)(tv_tiles(R) * ((R + zc - 1) / zc));
+}
 
 template <bool UPDATE>
 cudaError_t launch_tv(TvArgs a, cudaStream_t s)
 {
-    a.zc = tv_planes(a.R);
-    tv_kernel<UPDATE><<<tv_grid(a.R), kTvThreads, 0, s>>>(a);
+    a.zc = tv_planes<UPDATE>(a.R);
+    tv_kernel<UPDATE><<<tv_grid<UPDATE>(a.R), kTvThreads, 0, s>>>(a);
     note_launch();
     return cudaGetLastError();
 }
@@ -692,7 +696,7 @@ extern "C" ctdm_status ctdm_tape_create(int device, int R, const ctdm_cfloat *d_
     };
     t->TB = tile_lines(R);
     t->tiles = (long)R * R / t->TB;
-    const long parts = t->tiles > tv_grid(R) ? t->tiles : tv_grid(R);
+    const long tv = (long)tv_tiles(R) * ((R + 3) / 4), parts = t->tiles > tv ? t->tiles : tv;
     uint8_t *flags = nullptr;   // measured voxels, while the tape is built
     int *bc = nullptr;          // block counts, then offsets
     struct Scratch {
@@ -808,7 +812,7 @@ extern "C" ctdm_status ctdm_loss_grad(ctdm_tape *t, const ctdm_cfloat *d_V, doub
         a.eps2 = (float)eps * (float)eps;
         a.partial = t->red;
         e = launch_tv<false>(a, 0);
-        if (e == cudaSuccess) tv = sum_partials(t->red, tv_grid(t->R));
+        if (e == cudaSuccess) tv = sum_partials(t->red, tv_grid<false>(t->R));
     }
     if (e != cudaSuccess) return cuda_fail(e, "loss and gradient");
     if (loss) *loss = data + lambda * tv;
@@ -862,7 +866,7 @@ extern "C" ctdm_status ctdm_reconstruct_gradient_ex(ctdm_tape *t, int iterations
             GCK(launch_tv<true>(a, s), "update");
             if (h_loss) {
                 GCK(cudaStreamSynchronize(s), "loss");
-                loss += lambda * sum_partials(t->red, tv_grid(t->R));
+                loss += lambda * sum_partials(t->red, tv_grid<true>(t->R));
             }
             float2 *tmp = W;
             W = Wn;

@@ -258,24 +258,6 @@ constexpr int kTy = 8;   // rows (warps) per CTA
 // Voxels per lane for side R, tiles (rows of a CTA) per plane.
 constexpr int tv_vx(int R) { return R % 128 == 0 ? 4 : R / 32; }
 int tv_tiles(int R) { return (R / (32 * tv_vx(R))) * (R / kTy); }
-// Planes per march (at least 4) that make the grid's waves shortest: waves of `resident`
-// CTAs, each one plane longer than its own planes.  256^3 on 456 resident CTAs: 7 chunks of
-// 37 planes, one wave; chunks of 32 took a second wave for the last 56 CTAs, and twice as long.
-int tv_planes(int R, int resident)
-{
-    int best = R;
-    long cost = -1;
-    for (int zc = 4; zc <= R; zc++) {
-        const long ctas = (long)tv_tiles(R) * ((R + zc - 1) / zc);
-        const long c = (resident > 0 ? (ctas + resident - 1) / resident : ctas) * (zc + 1);
-        if (cost < 0 || c < cost) {
-            cost = c;
-            best = zc;
-        }
-    }
-    return best;
-}
-
 template <int VX>
 __device__ __forceinline__ void ld_vec(const float *__restrict__ p, float *v)
 {
@@ -411,7 +393,7 @@ template <bool STEP>
 cudaError_t launch_tv(const float *Vin, const float *gin, float *Vout, float *gout, const PocsBufs &b, cudaStream_t s)
 {
     auto k = tv_vx(b.R) == 4 ? tv_kernel<STEP, 4> : (tv_vx(b.R) == 2 ? tv_kernel<STEP, 2> : tv_kernel<STEP, 1>);
-    const int zc = tv_planes(b.R, wave_ctas(k, kThreads, 0));
+    const int zc = march_planes(b.R, tv_tiles(b.R), wave_ctas(k, kThreads, 0));
     k<<<(unsigned)(tv_tiles(b.R) * ((b.R + zc - 1) / zc)), kThreads, 0, s>>>(Vin, gin, Vout, gout, b.R, zc, b.tv_eps,
                                                                             b.ctl, b.part);
     note_launch();
