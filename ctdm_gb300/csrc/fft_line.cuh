@@ -145,13 +145,49 @@ __device__ __forceinline__ void dft3(float2 *a)
     a[2] = csub(m, t2);
 }
 
+// 6 = 2 x 3 without twiddles (prime factors: n = 3 n1 + 2 n2, k = 3 k1 + 4 k2 mod 6)
+template <bool INV>
+__device__ __forceinline__ void dft6(float2 *a)
+{
+    float2 p[3] = {a[0], a[2], a[4]}, q[3] = {a[3], a[5], a[1]};
+    dft3<INV>(p);
+    dft3<INV>(q);
+    a[0] = cadd(p[0], q[0]);
+    a[3] = csub(p[0], q[0]);
+    a[4] = cadd(p[1], q[1]);
+    a[1] = csub(p[1], q[1]);
+    a[2] = cadd(p[2], q[2]);
+    a[5] = csub(p[2], q[2]);
+}
+
+// 12 = 3 x 4 without twiddles (n = 4 n1 + 3 n2, k = 4 k1 + 9 k2 mod 12)
+template <bool INV>
+__device__ __forceinline__ void dft12(float2 *a)
+{
+    float2 b[4][3];
+#pragma unroll
+    for (int n2 = 0; n2 < 4; n2++) {
+#pragma unroll
+        for (int n1 = 0; n1 < 3; n1++) b[n2][n1] = a[(4 * n1 + 3 * n2) % 12];
+        dft3<INV>(b[n2]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 3; k1++) {
+        dft4<INV>(b[0][k1], b[1][k1], b[2][k1], b[3][k1]);
+#pragma unroll
+        for (int k2 = 0; k2 < 4; k2++) a[(4 * k1 + 9 * k2) % 12] = b[k2][k1];
+    }
+}
+
 template <int R, bool INV>
 __device__ __forceinline__ void dftR(float2 *a)
 {
     if constexpr (R == 2) dft2<INV>(a[0], a[1]);
     else if constexpr (R == 3) dft3<INV>(a);
     else if constexpr (R == 4) dft4<INV>(a[0], a[1], a[2], a[3]);
+    else if constexpr (R == 6) dft6<INV>(a);
     else if constexpr (R == 8) dft8<INV>(a);
+    else if constexpr (R == 12) dft12<INV>(a);
     else if constexpr (R == 16) dft16<INV>(a);
 }
 
@@ -162,6 +198,18 @@ template <int L, int LP, bool TF>
 struct Lay {
     static constexpr int LINE = TF ? L + L / 16 : LP;
     __device__ static __forceinline__ int at(int p) { return TF ? p + (p >> 4) : p; }
+    // at(p + r * S) - at(p) where that does not depend on p: p & 15 then leaves every
+    // step's carry into the next 16 points to r * S alone.  Written out because the
+    // compiler otherwise computes the shift for every point of a butterfly (the 512^2 plane
+    // pass held to 80 registers spilled 520 bytes a thread with that, 116 without).
+    __device__ static __forceinline__ constexpr int step(int rS) { return TF ? rS + (rS >> 4) : rS; }
+    // gathers: p = j + r * S
+    static constexpr bool gather_affine(int S) { return !TF || S % 16 == 0; }
+    // scatters: p = (j / S) * S * R + j % S + r * S
+    static constexpr bool scatter_affine(int S, int R)
+    {
+        return !TF || S % 16 == 0 || (16 % S == 0 && ((S * R) % 16 == 0 || 16 % (S * R) == 0));
+    }
 };
 
 // Register tile v[E], E = L / T, viewed as PER butterflies of R points.
@@ -174,7 +222,10 @@ __device__ __forceinline__ void gather(const float2 *buf, float2 *v, int b, int 
 #pragma unroll
     for (int q = 0; q < PER; q++)
 #pragma unroll
-        for (int r = 0; r < R; r++) v[q * R + r] = line[Y::at(t + T * q + r * NB)];
+        for (int r = 0; r < R; r++) {
+            if constexpr (Y::gather_affine(NB)) v[q * R + r] = line[Y::at(t + T * q) + Y::step(r * NB)];
+            else v[q * R + r] = line[Y::at(t + T * q + r * NB)];
+        }
 }
 
 template <int L, int T, bool INV, int NS, int R>
@@ -207,7 +258,10 @@ __device__ __forceinline__ void scatter(float2 *buf, const float2 *v, int b, int
         const int j = t + T * q;
         const int base = (j / NS) * NS * R + (j % NS);
 #pragma unroll
-        for (int r = 0; r < R; r++) line[Y::at(base + r * NS)] = v[q * R + r];
+        for (int r = 0; r < R; r++) {
+            if constexpr (Y::scatter_affine(NS, R)) line[Y::at(base) + Y::step(r * NS)] = v[q * R + r];
+            else line[Y::at(base + r * NS)] = v[q * R + r];
+        }
     }
 }
 
@@ -328,7 +382,10 @@ struct Ends {
     static constexpr int F = Plan<L>::F0, Rv = Plan<L>::RV0;
 };
 
-// Plan variants of the volume passes, chosen per pass by the autotuner.  Every
+// Plan variants of the volume passes, chosen per pass by the autotuner.  384 and 768 points
+// take three stages with a radix of 6 or 12 in the middle: with 4, 4, 8, 3 (8, 8, 4, 3) the
+// fourth exchange and its twiddles cost the 384^3 x pass 402 us per launch against 277, the
+// 768^3 x pass (8 lines) 3.71 ms against 2.35.  Every
 // stage's butterfly count L / R must be a multiple of T.
 template <int L, int V>
 struct PV;
@@ -336,12 +393,12 @@ template <int L>
 struct PV<L, 0> : Plan<L> {};
 template <> struct PV<256, 1> : PlanT<256, 8, 16, Radices<16, 16>, Radices<16, 16>> {};
 template <> struct PV<256, 2> : PlanT<256, 16, 32, Radices<8, 4, 8>, Radices<8, 4, 8>> {};
-template <> struct PV<384, 1> : PlanT<384, 16, 16, Radices<4, 4, 8, 3>, Radices<3, 8, 4, 4>> {};
-template <> struct PV<384, 2> : PlanT<384, 8, 16, Radices<4, 4, 8, 3>, Radices<3, 8, 4, 4>> {};
+template <> struct PV<384, 1> : PlanT<384, 16, 16, Radices<8, 6, 8>, Radices<8, 6, 8>> {};
+template <> struct PV<384, 2> : PlanT<384, 8, 16, Radices<8, 6, 8>, Radices<8, 6, 8>> {};
 template <> struct PV<512, 1> : PlanT<512, 16, 32, Radices<8, 8, 8>, Radices<8, 8, 8>> {};
 template <> struct PV<512, 2> : PlanT<512, 8, 32, Radices<8, 8, 8>, Radices<8, 8, 8>> {};
-template <> struct PV<768, 1> : PlanT<768, 8, 32, Radices<8, 8, 4, 3>, Radices<3, 4, 8, 8>> {};
-template <> struct PV<768, 2> : PlanT<768, 16, 32, Radices<8, 8, 4, 3>, Radices<3, 4, 8, 8>> {};
+template <> struct PV<768, 1> : PlanT<768, 8, 32, Radices<8, 12, 8>, Radices<8, 12, 8>> {};
+template <> struct PV<768, 2> : PlanT<768, 16, 32, Radices<8, 12, 8>, Radices<8, 12, 8>> {};
 
 // Point index of register slot i (butterfly q = i / R, point r = i % R) at the
 // register-resident end of a sequence whose end radix is R: j + r * (L / R).
