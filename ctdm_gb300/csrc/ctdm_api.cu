@@ -606,6 +606,9 @@ static long qpi_chunk(int N, int M, int A)
     return chunk > A ? A : chunk;
 }
 
+// A single shared background rides along with the first chunk of holograms (one launch for
+// both in every pass but the last; at 31 x 1024^2 the background's own passes took 22 of 191
+// us); per-angle backgrounds are transformed here.
 static ctdm_status qpi_setup(ctdm_ctx *c, int N, int M, int A, const float *bg, int bg_per_angle,
                              const int *carrier_in, cudaStream_t s)
 {
@@ -613,7 +616,6 @@ static ctdm_status qpi_setup(ctdm_ctx *c, int N, int M, int A, const float *bg, 
     if (!ok_length(M) || M > N) return invalid("window side %d unsupported", M);
     if (A < 1) return invalid("no angles");
     CK(ensure(c, B_CARRIER, sizeof(int) * 3), "alloc carrier");
-    CK(ensure(c, B_KEY, sizeof(unsigned long long)), "alloc key");
     int *car = B<int>(c, B_CARRIER);
     if (carrier_in && carrier_in[0] >= 0 && carrier_in[1] >= 0 && carrier_in[2] >= 0) {
         if (carrier_in[1] - M / 2 < 0 || carrier_in[1] + M / 2 > N || carrier_in[0] - M / 2 < 0 ||
@@ -622,43 +624,52 @@ static ctdm_status qpi_setup(ctdm_ctx *c, int N, int M, int A, const float *bg, 
         CK(set_carrier(car, carrier_in[0], carrier_in[1], carrier_in[2], s), "set carrier");
     } else {
         CK(ensure(c, B_SCRATCH, sizeof(float2) * N * N), "alloc carrier scratch");
+        if (!c->buf[B_KEY]) {   // the search leaves its state zero
+            CK(ensure(c, B_KEY, 2 * sizeof(unsigned long long)), "alloc key");
+            CK(cudaMemsetAsync(c->buf[B_KEY], 0, 2 * sizeof(unsigned long long), s), "clear key");
+        }
         CK(qpi_find_carrier(bg, N, B<float2>(c, B_SCRATCH), B<unsigned long long>(c, B_KEY), car, s),
            "carrier search");
     }
-    const long chunk = qpi_chunk(N, M, A);
+    const long chunk = qpi_chunk(N, M, A) + (bg_per_angle ? 0 : 1);
     const long mm = (long)M * M, nn = (long)N * N;
     CK(ensure(c, B_T1, sizeof(float2) * chunk * N * M), "alloc T1");
     CK(ensure(c, B_S, sizeof(float2) * chunk * mm), "alloc S");
     const int nbg = bg_per_angle ? A : 1;
     CK(ensure(c, B_BGF, sizeof(float2) * nbg * mm), "alloc BG field");
-    for (long a0 = 0; a0 < nbg; a0 += chunk) {
+    for (long a0 = 0; bg_per_angle && a0 < nbg; a0 += chunk) {
         const int ac = (int)std::min<long>(chunk, nbg - a0);
-        CK(qpi_forward_window(bg + a0 * nn, 4, ac, N, M, car, B<float2>(c, B_T1), B<float2>(c, B_S), s),
+        CK(qpi_forward_window(nullptr, 0, bg + a0 * nn, 4, ac, N, M, car, B<float2>(c, B_T1), B<float2>(c, B_S), s),
            "qpi bg fwd");
-        CK(qpi_inverse_window(B<float2>(c, B_S), ac, M, car, B<float2>(c, B_BGF) + a0 * mm, nullptr, 0, nullptr,
-                              nullptr, s),
+        CK(qpi_inverse_rows(B<float2>(c, B_S), ac, M, car, s), "qpi bg inv");
+        CK(qpi_inverse_cols(B<float2>(c, B_S), ac, M, car, B<float2>(c, B_BGF) + a0 * mm, true, nullptr, 0, nullptr,
+                            nullptr, s),
            "qpi bg inv");
     }
     return CTDM_OK;
 }
 
 // Second part: phase and amplitude of angles [first, first + count) (holo: the whole
-// stack; the background fields of qpi_setup).
+// stack; the background fields of qpi_setup, or with first = 0 the shared background bg).
 // holo: the stack, bpc bytes per pixel (4 float, 2 / 1 camera counts)
 static ctdm_status qpi_angles(ctdm_ctx *c, int N, int M, int A, int first, int count, const void *holo, int bpc,
-                              int bg_per_angle, float *phase, float *amp, cudaStream_t s)
+                              const float *bg, int bg_per_angle, float *phase, float *amp, cudaStream_t s)
 {
     const long chunk = qpi_chunk(N, M, A);
     const long mm = (long)M * M, nn = (long)N * N;
     const int *car = B<int>(c, B_CARRIER);
     for (long a0 = first; a0 < first + count; a0 += chunk) {
-        const int ac = (int)std::min<long>(chunk, first + count - a0);
-        CK(qpi_forward_window(static_cast<const char *>(holo) + (size_t)bpc * a0 * nn, bpc, ac, N, M, car,
-                              B<float2>(c, B_T1), B<float2>(c, B_S), s),
+        const int ac = (int)std::min<long>(chunk, first + count - a0), nbg = a0 == 0 && !bg_per_angle ? 1 : 0;
+        float2 *S = B<float2>(c, B_S);
+        CK(qpi_forward_window(bg, nbg, static_cast<const char *>(holo) + (size_t)bpc * a0 * nn, bpc, ac, N, M, car,
+                              B<float2>(c, B_T1), S, s),
            "qpi fwd");
+        CK(qpi_inverse_rows(S, nbg + ac, M, car, s), "qpi inv");
+        if (nbg)
+            CK(qpi_inverse_cols(S, 1, M, car, B<float2>(c, B_BGF), true, nullptr, 0, nullptr, nullptr, s), "qpi bg inv");
         const float2 *bgf = B<float2>(c, B_BGF) + (bg_per_angle ? a0 * mm : 0);
-        CK(qpi_inverse_window(B<float2>(c, B_S), ac, M, car, nullptr, bgf, bg_per_angle ? mm : 0, phase + a0 * mm,
-                              amp + a0 * mm, s),
+        CK(qpi_inverse_cols(S + nbg * mm, ac, M, car, nullptr, false, bgf, bg_per_angle ? mm : 0, phase + a0 * mm,
+                            amp + a0 * mm, s),
            "qpi inv");
     }
     return CTDM_OK;
@@ -669,7 +680,7 @@ static ctdm_status do_qpi(ctdm_ctx *c, int N, int M, int A, const float *holo, c
 {
     ctdm_status st = qpi_setup(c, N, M, A, bg, bg_per_angle, carrier_in, s);
     if (st != CTDM_OK) return st;
-    return qpi_angles(c, N, M, A, 0, A, holo, 4, bg_per_angle, phase, amp, s);
+    return qpi_angles(c, N, M, A, 0, A, holo, 4, bg, bg_per_angle, phase, amp, s);
 }
 
 // Scale of the z lines that the loop starts from.
@@ -780,29 +791,24 @@ static ctdm_status do_qpi_b(ctdm_ctx *c, int N, int A, const float *holo, const 
     if (N < 64 || N > 2048 || (N & (N - 1))) return invalid("hologram side %d unsupported", N);
     if (A < 1) return invalid("no angles");
     const int M = N / 4;
-    const long mm = (long)M * M, nn = (long)N * N;
+    const long mm = (long)M * M;
     CK(ensure(c, B_CARRIER, sizeof(int) * 3), "alloc carrier");
     int *car = B<int>(c, B_CARRIER);
     if (center_in && center_in[0] >= 0 && center_in[1] >= 0) {
         if (center_in[0] >= N || center_in[1] >= N) return invalid("carrier column outside the spectrum");
         CK(set_carrier(car, center_in[0], center_in[1], -1, s), "set carrier");
     } else {
-        CK(ensure(c, B_QMAG, sizeof(float) * (N / 4) * N), "alloc histogram scratch");
-        CK(set_carrier(car, 0, 0, -1, s), "reset carrier");
-        // frame 1 of sequence1DFFT: the SP frame's own column first, then the background's
-        CK(qpib_spectrum_center(holo, N, B<float>(c, B_QMAG), car + 1, s), "carrier column (frame 1)");
-        CK(qpib_spectrum_center(bg, N, B<float>(c, B_QMAG), car, s), "carrier column (background)");
+        CK(ensure(c, B_QMAG, 2 * sizeof(float) * (N / 4) * N), "alloc histogram scratch");
+        // frame 1 of sequence1DFFT: the SP frame's own column and the background's
+        CK(qpib_centers(bg, holo, N, B<float>(c, B_QMAG), car, s), "carrier columns");
     }
     const int nbg = bg_per_angle ? A : 1;
-    const int rows = A > nbg ? A : nbg;
-    CK(ensure(c, B_T1, sizeof(float2) * rows * mm), "alloc window rows");
+    CK(ensure(c, B_T1, sizeof(float2) * (nbg + A) * mm), "alloc window rows");
     CK(ensure(c, B_BGF, sizeof(float2) * nbg * mm), "alloc BG field");
     float2 *T = B<float2>(c, B_T1), *bgf = B<float2>(c, B_BGF);
-    CK(qpib_window(bg, nbg, N, car, T, s), "qpi B background window");
-    CK(qpib_inverse(T, nbg, M, bgf, nullptr, 0, nullptr, nullptr, s), "qpi B background field");
-    CK(qpib_window(holo, 1, N, car + 1, T, s), "qpi B window (frame 1)");
-    if (A > 1) CK(qpib_window(holo + nn, A - 1, N, car, T + mm, s), "qpi B window");
-    CK(qpib_inverse(T, A, M, nullptr, bgf, bg_per_angle ? mm : 0, phase, amp, s), "qpi B fields");
+    CK(qpib_window(bg, nbg, holo, A, N, car, T, s), "qpi B windows");
+    CK(qpib_inverse(T, nbg, M, bgf, true, nullptr, 0, nullptr, nullptr, s), "qpi B background field");
+    CK(qpib_inverse(T + nbg * mm, A, M, nullptr, false, bgf, bg_per_angle ? mm : 0, phase, amp, s), "qpi B fields");
     return CTDM_OK;
 }
 
@@ -943,7 +949,7 @@ static ctdm_status pipeline_core(ctdm_ctx *c, const ctdm_params *p, int A, int M
         if (!alg_b) {
             if (feed) CK(cudaStreamWaitEvent(s, feed->ready[k], 0), "wait for holograms");
             const bool cnt = feed && feed->counts;
-            st = qpi_angles(c, N, M, A, a0, ac, cnt ? feed->counts : d_holo, cnt ? feed->bpc : 4, p->bg_per_angle,
+            st = qpi_angles(c, N, M, A, a0, ac, cnt ? feed->counts : d_holo, cnt ? feed->bpc : 4, d_bg, p->bg_per_angle,
                             B<float>(c, B_PHASE), B<float>(c, B_AMP),
                             s);
             if (st != CTDM_OK) return st;
@@ -1065,9 +1071,9 @@ size_t workspace_bytes(const ctdm_params *p, int A, int M)
     if (p->run_goldstein || p->unwrap_method == CTDM_METHOD_GOLDSTEIN)
         b += (size_t)A * mm * (1 + 1 + 4 + 1 + 20 + 1) + 4 * (size_t)A;   // charges, cuts, out, state, lists, work
     if (p->unwrap_method == CTDM_METHOD_FAST) b += 4 * (size_t)A * mm + 96 * mm;
-    const size_t chunk = (size_t)qpi_chunk((int)N, M, A);
-    b += chunk * N * M * 8 + chunk * mm * 8 + (p->bg_per_angle ? (size_t)A : 1) * mm * 8 + N * N * 8 + 64;
-    if (p->qpi_method == CTDM_QPI_B) b += N * N + N * N * 2;          // column histogram scratch, window rows
+    const size_t chunk = (size_t)qpi_chunk((int)N, M, A) + 1, nbg = p->bg_per_angle ? (size_t)A : 1;
+    b += chunk * N * M * 8 + chunk * mm * 8 + nbg * mm * 8 + N * N * 8 + 64;
+    if (p->qpi_method == CTDM_QPI_B) b += N * N * 2 + (A + nbg) * mm * 8;   // column histogram scratch, window rows
     b += 9 * r3 + 4 * rr;                                    // packed samples, masks, prefixes (tiles of >= 8)
     if (p->accelerated && p->iterations > 0) b += 8 * r3;    // the accelerated loop's iterate
     b += sizeof(AngleGeom) * (size_t)A + 4096;
@@ -1759,13 +1765,15 @@ extern "C" void extractQPI_AlgorithmA(ctdm_cfloat *SP, ctdm_cfloat *BG, ctdm_cfl
         if (e != cudaSuccess) { cuda_fail(e, "extractQPI_AlgorithmA carrier"); return; }
         g_qpia_carrier[c->device] = {host[0], host[1], host[2]};
     }
-    e = cudaMemcpyAsync(cuBG_FFT, c->buf[B_BGF], sizeof(float2) * mm, cudaMemcpyDeviceToDevice, 0);
+    const int *car = B<int>(c, B_CARRIER);
+    float2 *S = B<float2>(c, B_S);
+    e = qpi_forward_window(B<float>(c, B_BG), 1, B<float>(c, B_HOLO), 4, 1, N, M, car, B<float2>(c, B_T1), S, 0);
+    if (e == cudaSuccess) e = qpi_inverse_rows(S, 2, M, car, 0);
     if (e == cudaSuccess)
-        e = qpi_forward_window(B<float>(c, B_HOLO), 4, 1, N, M, B<int>(c, B_CARRIER), B<float2>(c, B_T1),
-                               B<float2>(c, B_S), 0);
+        e = qpi_inverse_cols(S, 1, M, car, reinterpret_cast<float2 *>(cuBG_FFT), false, nullptr, 0, nullptr, nullptr, 0);
     if (e == cudaSuccess)
-        e = qpi_inverse_window(B<float2>(c, B_S), 1, M, B<int>(c, B_CARRIER), reinterpret_cast<float2 *>(cuSP_FFT),
-                               nullptr, 0, nullptr, nullptr, 0);
+        e = qpi_inverse_cols(S + mm, 1, M, car, reinterpret_cast<float2 *>(cuSP_FFT), false, nullptr, 0, nullptr,
+                             nullptr, 0);
     if (e != cudaSuccess) { cuda_fail(e, "extractQPI_AlgorithmA"); return; }
     finish("extractQPI_AlgorithmA");
 }
@@ -1788,7 +1796,8 @@ extern "C" void extractQPI_AlgorithmB(float *SP, float *BG, ctdm_cfloat *cuSP_FF
     const long nn = (long)N * N;
     if (wait_host(c) != CTDM_OK) return;   // host-buffer calls in flight still own B_HOLO / B_BG
     if (ensure(c, B_HOLO, sizeof(float) * nn) != cudaSuccess || ensure(c, B_BG, sizeof(float) * nn) != cudaSuccess ||
-        ensure(c, B_T1, sizeof(float2) * M * M) != cudaSuccess || ensure(c, B_QMAG, sizeof(float) * M * N) != cudaSuccess ||
+        ensure(c, B_T1, 2 * sizeof(float2) * M * M) != cudaSuccess ||
+        ensure(c, B_QMAG, 2 * sizeof(float) * M * N) != cudaSuccess ||
         ensure(c, B_CARRIER, sizeof(int) * 3) != cudaSuccess) {
         cuda_fail(cudaErrorMemoryAllocation, "extractQPI_AlgorithmB");
         return;
@@ -1802,8 +1811,7 @@ extern "C" void extractQPI_AlgorithmB(float *SP, float *BG, ctdm_cfloat *cuSP_FF
     cudaError_t e = cudaSuccess;
     if (frame == 1) {
         // the SP frame's own column, then the background's, which later frames keep
-        e = qpib_spectrum_center(B<float>(c, B_HOLO), N, B<float>(c, B_QMAG), car + 1, 0);
-        if (e == cudaSuccess) e = qpib_spectrum_center(B<float>(c, B_BG), N, B<float>(c, B_QMAG), car, 0);
+        e = qpib_centers(B<float>(c, B_BG), B<float>(c, B_HOLO), N, B<float>(c, B_QMAG), car, 0);
         int host[2] = {0, 0};
         if (e == cudaSuccess) e = cudaMemcpy(host, car, sizeof(int) * 2, cudaMemcpyDeviceToHost);
         if (e == cudaSuccess) g_qpib_column[c->device] = host[0];
@@ -1813,10 +1821,11 @@ extern "C" void extractQPI_AlgorithmB(float *SP, float *BG, ctdm_cfloat *cuSP_FF
         e = set_carrier(car, it->second, it->second, -1, 0);
     }
     float2 *T = B<float2>(c, B_T1);
-    if (e == cudaSuccess) e = qpib_window(B<float>(c, B_HOLO), 1, N, car + 1, T, 0);
-    if (e == cudaSuccess) e = qpib_inverse(T, 1, M, reinterpret_cast<float2 *>(cuSP_FFT), nullptr, 0, nullptr, nullptr, 0);
-    if (e == cudaSuccess) e = qpib_window(B<float>(c, B_BG), 1, N, car, T, 0);
-    if (e == cudaSuccess) e = qpib_inverse(T, 1, M, reinterpret_cast<float2 *>(cuBG_FFT), nullptr, 0, nullptr, nullptr, 0);
+    if (e == cudaSuccess) e = qpib_window(B<float>(c, B_BG), 1, B<float>(c, B_HOLO), 1, N, car, T, 0);
+    if (e == cudaSuccess)
+        e = qpib_inverse(T, 1, M, reinterpret_cast<float2 *>(cuBG_FFT), false, nullptr, 0, nullptr, nullptr, 0);
+    if (e == cudaSuccess)
+        e = qpib_inverse(T + (long)M * M, 1, M, reinterpret_cast<float2 *>(cuSP_FFT), false, nullptr, 0, nullptr, nullptr, 0);
     if (e != cudaSuccess) { cuda_fail(e, "extractQPI_AlgorithmB"); return; }
     finish("extractQPI_AlgorithmB");
 }

@@ -267,13 +267,16 @@ __device__ __forceinline__ void scatter(float2 *buf, const float2 *v, int b, int
 
 // Barrier between the shared-memory exchanges of a transform.  Under the row mapping a
 // line's T threads are consecutive, so with T dividing 32 a line lies inside one warp and
-// touches only its own slots: a warp barrier orders its exchanges.  The column mapping
-// spreads a line over the CTA and needs the CTA barrier.  (Exchanges with data written
+// touches only its own slots: a warp barrier orders its exchanges.  A line of 2 or 4 whole
+// warps has a named barrier of its own (1 + b), so that the CTA's lines do not wait for each
+// other.  The column mapping spreads a line over the CTA and needs the CTA barrier.  (Exchanges with data written
 // or read by another mapping, GATHER0 / SCATTER_LAST, keep the CTA barrier.)
 template <bool TF, int T, bool LOCAL>
-__device__ __forceinline__ void line_sync()
+__device__ __forceinline__ void line_sync(int b)
 {
     if constexpr (TF && LOCAL && T <= 32 && (32 % T) == 0) __syncwarp();
+    else if constexpr (TF && LOCAL && (T == 64 || T == 128))
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + b), "n"(T) : "memory");  
     else __syncthreads();
 }
 
@@ -287,12 +290,12 @@ __device__ __forceinline__ void stages(float2 *buf, float2 *v, const float2 *__r
     constexpr bool last = (sizeof...(REST) == 0);
     if constexpr (!first || GATHER0) {
         gather<L, T, LP, R, TF>(buf, v, b, t);
-        line_sync<TF, T, !(first && GATHER0)>();
+        line_sync<TF, T, !(first && GATHER0)>(b);
     }
     compute<L, T, INV, NS, R>(v, tw, t);
     if constexpr (!last || SCATTER_LAST) {
         scatter<L, T, LP, NS, R, TF>(buf, v, b, t);
-        line_sync<TF, T, !(last && SCATTER_LAST)>();
+        line_sync<TF, T, !(last && SCATTER_LAST)>(b);
     }
     if constexpr (!last) stages<L, T, LP, INV, GATHER0, SCATTER_LAST, TF, NS * R, REST...>(buf, v, tw, b, t);
 }
@@ -320,6 +323,7 @@ struct PlanT<L_, B_, T_, Radices<FW...>, Radices<RV...>> {
     static constexpr int E = L / T;
     static constexpr int F0 = FirstOf<FW...>::v, RV0 = FirstOf<RV...>::v;
     static_assert(E * T == L, "threads per line must divide the length");
+    static_assert(T < 64 || B <= 15, "one named barrier per line of more than a warp");
     template <bool INV, bool GATHER0, bool SCATTER_LAST>
     __device__ static __forceinline__ void seq(float2 *buf, float2 *v, const float2 *tw)
     {

@@ -17,6 +17,7 @@
 
 #include "fft_line.cuh"
 #include "kernels_front.cuh"
+#include "line_kernels.cuh"
 
 namespace ctdm {
 
@@ -36,7 +37,10 @@ static cudaError_t set_smem(K kernel, size_t smem)
 // j >= start of the quadrant-swapped spectrum, first maximum in raster order.
 // Packed key: (bits of |X|^2) << 32 | ~(raster index) so that atomicMax picks the
 // largest magnitude and, among equal ones, the smallest index.
-__global__ void carrier_argmax_kernel(const float2 *__restrict__ spec, int N, int start, unsigned long long *key)
+// state: {key, CTAs done}, zero before the launch; the last CTA writes the carrier and zeroes
+// it for the next call.
+__global__ void __launch_bounds__(256) carrier_argmax_kernel(const float2 *__restrict__ spec, int N, int start,
+                                                             unsigned long long *state, int *carrier)
 {
     unsigned long long best = 0ull;
     const long total = (long)(N - start) * N;
@@ -53,41 +57,50 @@ __global__ void carrier_argmax_kernel(const float2 *__restrict__ spec, int N, in
         unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
         if (other > best) best = other;
     }
-    if ((threadIdx.x & 31) == 0) atomicMax(key, best);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&state[0], best);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&state[1], 1ull) == gridDim.x - 1) {
+        __threadfence();
+        const unsigned idx = ~(unsigned)(atomicExch(&state[0], 0ull) & 0xffffffffull);
+        const int r = (int)(idx / (unsigned)N), c = (int)(idx % (unsigned)N);
+        carrier[0] = r;
+        carrier[1] = c;
+        carrier[2] = abs(r - N / 2) / 3;
+        state[1] = 0ull;
+    }
 }
 
-__global__ void carrier_finish_kernel(const unsigned long long *key, int N, int *carrier)
+// Forward row transforms of real rows (the image is read as it is).
+struct LoadRealRow {
+    const float *p;
+    __device__ __forceinline__ float2 operator()(long i) const { return make_float2(__ldg(p + i), 0.f); }
+};
+template <int L>
+static cudaError_t rows_real_launch(const float *src, float2 *dst, long nlines, cudaStream_t s)
 {
-    const unsigned idx = ~(unsigned)(*key & 0xffffffffull);
-    const int r = (int)(idx / (unsigned)N), c = (int)(idx % (unsigned)N);
-    carrier[0] = r;
-    carrier[1] = c;
-    carrier[2] = abs(r - N / 2) / 3;
+    return rows_fn_launch<RowPlan<L>, false>(LoadRealRow{src}, StoreScaled{dst, 1.0f}, nlines, s);
 }
-
-__global__ void real_to_complex_kernel(const float *__restrict__ in, float2 *out, long n)
+static cudaError_t fft_rows_real(const float *src, float2 *dst, int L, long nlines, cudaStream_t s)
 {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        out[i] = make_float2(in[i], 0.f);
+    CTDM_DISPATCH_L(L, rows_real_launch, src, dst, nlines, s)
 }
 
-cudaError_t qpi_find_carrier(const float *bg, int N, float2 *scratch, unsigned long long *key, int *carrier,
+cudaError_t qpi_find_carrier(const float *bg, int N, float2 *scratch, unsigned long long *state, int *carrier,
                              cudaStream_t s)
 {
-    const long n2 = (long)N * N;
-    real_to_complex_kernel<<<1024, 256, 0, s>>>(bg, scratch, n2); note_launch();
-    cudaError_t e = fft_rows(scratch, N, N, false, s);
+    cudaError_t e = fft_rows_real(bg, scratch, N, N, s);
     if (e == cudaSuccess) e = fft_cols(scratch, N, N, N, 0, N, false, s);
     if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(key, 0, sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
-    carrier_argmax_kernel<<<256, 256, 0, s>>>(scratch, N, (600 * N) / 1024, key); note_launch();
-    carrier_finish_kernel<<<1, 1, 0, s>>>(key, N, carrier); note_launch();
+    carrier_argmax_kernel<<<256, 256, 0, s>>>(scratch, N, (600 * N) / 1024, state, carrier); note_launch();
     return cudaGetLastError();
 }
 
 // ------------------------------------------------------------ forward row pass
-// holo: A holograms N x N (float, [a][y][x]); T1: A x N x M complex ([a][y][m]).
+// bg: background holograms (bgpairs row pairs; their T1 rows come first), holo: A holograms
+// N x N ([a][y][x]); T1: N x M complex per hologram ([a][y][m]).
 // Column m of the window is spectrum column k = (c - N/2 + m - M/2) mod N of the
 // unshifted transform (the quadrant swap folded into the index).
 //
@@ -107,8 +120,8 @@ template <> struct QRows<2048> : fftl::PlanT<2048, 2, 128, fftl::Radices<16, 16,
 // QPI A over 121 x 1024^2 holograms.
 template <int N, class T>
 __global__ void __launch_bounds__(QRows<N>::THREADS, 1024 / QRows<N>::THREADS)
-    qpi_rows_kernel(const T *__restrict__ holo, float2 *T1, const int *__restrict__ carrier, long npairs, int M,
-                    const float2 *__restrict__ tw)
+    qpi_rows_kernel(const float *__restrict__ bg, const T *__restrict__ holo, float2 *T1,
+                    const int *__restrict__ carrier, long bgpairs, long npairs, int M, const float2 *__restrict__ tw)
 {
     using P = QRows<N>;
     using Y = fftl::Lay<N, P::LP, true>;
@@ -117,12 +130,21 @@ __global__ void __launch_bounds__(QRows<N>::THREADS, 1024 / QRows<N>::THREADS)
     const int t = threadIdx.x % P::T, b = threadIdx.x / P::T;
     const long q = (long)blockIdx.x * P::B + b;   // pair q covers rows 2q, 2q+1 of the stack
     const bool ok = q < npairs;
-    const T *r0 = holo + (ok ? 2 * q : 0) * N;
     float2 v[P::E];
+    if (q < bgpairs) {   // the same for the whole line: pairs of the background come first
+        const float *r0 = bg + 2 * q * N;
 #pragma unroll
-    for (int i = 0; i < P::E; i++) {
-        const int p = fftl::slot_pos<N, P::T, P::F0>(i, t);
-        v[i] = ok ? make_float2((float)__ldcs(&r0[p]), (float)__ldcs(&r0[N + p])) : make_float2(0.f, 0.f);
+        for (int i = 0; i < P::E; i++) {
+            const int p = fftl::slot_pos<N, P::T, P::F0>(i, t);
+            v[i] = make_float2(__ldcs(&r0[p]), __ldcs(&r0[N + p]));
+        }
+    } else {
+        const T *r0 = holo + (ok ? 2 * (q - bgpairs) : 0) * N;
+#pragma unroll
+        for (int i = 0; i < P::E; i++) {
+            const int p = fftl::slot_pos<N, P::T, P::F0>(i, t);
+            v[i] = ok ? make_float2((float)__ldcs(&r0[p]), (float)__ldcs(&r0[N + p])) : make_float2(0.f, 0.f);
+        }
     }
     P::template seq_row<false>(buf, v, tw);
     float2 *line = buf + b * Y::LINE;
@@ -256,13 +278,29 @@ __global__ void __launch_bounds__(Plan<M>::THREADS) qpi_rows_inv_kernel(float2 *
 // Lines are the M columns of each M x M spectrum (rows already inverse
 // transformed; the rows outside the radius box are zero and not read).  Epilogue:
 // x 1/M^2 and conjugate (scaleFFT2D), then either store the complex field
-// (background) or the phase arg BG - arg SP and amplitude |SP|/|BG| with NaN/inf -> 0
-// (calcWrapPhase).
+// (background; polar: as its argument and modulus, which every frame's epilogue needs) or
+// the phase arg BG - arg SP and amplitude |SP|/|BG| with NaN/inf -> 0 (calcWrapPhase).
+
+// Argument and modulus of a background value, as calcWrapPhase takes them.
+__device__ __forceinline__ float2 to_polar(float2 g)
+{
+    return make_float2(atan2f(g.y, g.x), sqrtf(g.x * g.x + g.y * g.y));
+}
+// bg: to_polar of the background.
+__device__ __forceinline__ void wrap_phase(float2 v, float2 bg, float &ph, float &am)
+{
+    ph = bg.x - atan2f(v.y, v.x);
+    if (isnan(ph) || isinf(ph)) ph = 0.f;
+    am = sqrtf(v.x * v.x + v.y * v.y) / bg.y;
+    if (isnan(am) || isinf(am)) am = 0.f;
+}
+
 template <int M>
 __global__ void __launch_bounds__(Plan<M>::THREADS) qpi_final_kernel(const float2 *__restrict__ S, long nlines,
                                                                     const int *__restrict__ carrier,
-                                                                    float2 *field_out, const float2 *__restrict__ bgf,
-                                                                    long bg_stride, float *phase, float *amp,
+                                                                    float2 *field_out, bool polar,
+                                                                    const float2 *__restrict__ bgf, long bg_stride,
+                                                                    float *phase, float *amp,
                                                                     const float2 *__restrict__ tw)
 {
     using P = Plan<M>;
@@ -277,55 +315,56 @@ __global__ void __launch_bounds__(Plan<M>::THREADS) qpi_final_kernel(const float
     const long mm = (long)M * M;
     const float2 *src = S + a * mm + x;
     const int rad = __ldg(&carrier[2]);
-    for (int p = t; p < M; p += P::T)
-        buf[b * P::LP + p] = ok && (p <= rad || p >= M - rad) ? src[(long)p * M] : make_float2(0.f, 0.f);
-    __syncthreads();
-    P::template run<true>(buf, tw);
+    float2 v[P::E];
+#pragma unroll
+    for (int i = 0; i < P::E; i++) {
+        const int p = fftl::slot_pos<M, P::T, P::F0>(i, t);
+        v[i] = ok && (p <= rad || p >= M - rad) ? src[(long)p * M] : make_float2(0.f, 0.f);
+    }
+    P::template seq<true, false, false>(buf, v, tw);
     if (!ok) return;
     const float sc = 1.0f / (float)mm;
-    for (int y = t; y < M; y += P::T) {
-        const float2 raw = buf[b * P::LP + y];
-        const float2 v = make_float2(raw.x * sc, -raw.y * sc);
-        const long o = a * mm + x + (long)M * y;
+#pragma unroll
+    for (int i = 0; i < P::E; i++) {
+        const long o = x + (long)M * fftl::slot_pos<M, P::T, P::RV0>(i, t);
+        const float2 f = make_float2(v[i].x * sc, -v[i].y * sc);
         if (field_out) {
-            field_out[o] = v;
+            field_out[a * mm + o] = polar ? to_polar(f) : f;
         } else {
-            const float2 g = bgf[a * bg_stride + x + (long)M * y];
-            float ph = atan2f(g.y, g.x) - atan2f(v.y, v.x);
-            if (isnan(ph) || isinf(ph)) ph = 0.f;
-            float am = sqrtf(v.x * v.x + v.y * v.y) / sqrtf(g.x * g.x + g.y * g.y);
-            if (isnan(am) || isinf(am)) am = 0.f;
-            phase[o] = ph;
-            amp[o] = am;
+            float ph, am;
+            wrap_phase(f, bgf[a * bg_stride + o], ph, am);
+            phase[a * mm + o] = ph;
+            amp[a * mm + o] = am;
         }
     }
 }
 
 template <int N, class T>
-static cudaError_t qpi_rows_launch(const T *holo, long npairs, int M, const int *carrier, float2 *T1, cudaStream_t s)
+static cudaError_t qpi_rows_launch(const float *bg, int nbg, const T *holo, int A, int M, const int *carrier,
+                                   float2 *T1, cudaStream_t s)
 {
     using PR = QRows<N>;
     const size_t smem_r = fftl::plan_smem_row<PR>();
+    const long bgpairs = (long)nbg * N / 2, npairs = bgpairs + (long)A * N / 2;
     cudaError_t e = set_smem<N>(qpi_rows_kernel<N, T>, smem_r);
     if (e != cudaSuccess) return e;
-    qpi_rows_kernel<N, T><<<(unsigned)((npairs + PR::B - 1) / PR::B), PR::THREADS, smem_r, s>>>(holo, T1, carrier,
-                                                                                              npairs, M, twiddles(N));
+    qpi_rows_kernel<N, T><<<(unsigned)((npairs + PR::B - 1) / PR::B), PR::THREADS, smem_r, s>>>(
+        bg, holo, T1, carrier, bgpairs, npairs, M, twiddles(N));
     note_launch();
     return cudaGetLastError();
 }
 
 template <int N>
-static cudaError_t qpi_fwd_launch(const void *holo, int bpc, int A, int M, const int *carrier, float2 *T1, float2 *S,
-                                  cudaStream_t s)
+static cudaError_t qpi_fwd_launch(const float *bg, int nbg, const void *holo, int bpc, int A, int M,
+                                  const int *carrier, float2 *T1, float2 *S, cudaStream_t s)
 {
-    const long npairs = (long)A * N / 2;
     cudaError_t e;
-    if (bpc == 2) e = qpi_rows_launch<N>(static_cast<const uint16_t *>(holo), npairs, M, carrier, T1, s);
-    else if (bpc == 1) e = qpi_rows_launch<N>(static_cast<const uint8_t *>(holo), npairs, M, carrier, T1, s);
-    else e = qpi_rows_launch<N>(static_cast<const float *>(holo), npairs, M, carrier, T1, s);
+    if (bpc == 2) e = qpi_rows_launch<N>(bg, nbg, static_cast<const uint16_t *>(holo), A, M, carrier, T1, s);
+    else if (bpc == 1) e = qpi_rows_launch<N>(bg, nbg, static_cast<const uint8_t *>(holo), A, M, carrier, T1, s);
+    else e = qpi_rows_launch<N>(bg, nbg, static_cast<const float *>(holo), A, M, carrier, T1, s);
     if (e != cudaSuccess) return e;
     using PC = QCols<N>;
-    const long nl = (long)A * M;
+    const long nl = (long)(nbg + A) * M;
     const size_t smem = fftl::plan_smem<PC>();
     e = set_smem<N>(qpi_cols_kernel<N>, smem);
     if (e != cudaSuccess) return e;
@@ -335,8 +374,7 @@ static cudaError_t qpi_fwd_launch(const void *holo, int bpc, int A, int M, const
 }
 
 template <int M>
-static cudaError_t qpi_inv_launch(float2 *S, int A, const int *carrier, float2 *field_out, const float2 *bgf,
-                                  long bg_stride, float *phase, float *amp, cudaStream_t s)
+static cudaError_t qpi_inv_rows_launch(float2 *S, int A, const int *carrier, cudaStream_t s)
 {
     using P = Plan<M>;
     const long nl = (long)A * M;
@@ -345,25 +383,39 @@ static cudaError_t qpi_inv_launch(float2 *S, int A, const int *carrier, float2 *
     if (e != cudaSuccess) return e;
     qpi_rows_inv_kernel<M><<<(unsigned)((nl + P::B - 1) / P::B), P::THREADS, smem_r, s>>>(S, nl, carrier,
                                                                                          twiddles(M)); note_launch();
+    return cudaGetLastError();
+}
+
+template <int M>
+static cudaError_t qpi_inv_cols_launch(const float2 *S, int A, const int *carrier, float2 *field_out, bool polar,
+                                       const float2 *bgf, long bg_stride, float *phase, float *amp, cudaStream_t s)
+{
+    using P = Plan<M>;
+    const long nl = (long)A * M;
     const size_t smem = fftl::smem_bytes<M>();
-    e = set_smem<M>(qpi_final_kernel<M>, smem);
+    cudaError_t e = set_smem<M>(qpi_final_kernel<M>, smem);
     if (e != cudaSuccess) return e;
-    qpi_final_kernel<M><<<(unsigned)((nl + P::B - 1) / P::B), P::THREADS, smem, s>>>(S, nl, carrier, field_out, bgf,
-                                                                                    bg_stride, phase, amp, twiddles(M));
+    qpi_final_kernel<M><<<(unsigned)((nl + P::B - 1) / P::B), P::THREADS, smem, s>>>(
+        S, nl, carrier, field_out, polar, bgf, bg_stride, phase, amp, twiddles(M));
     note_launch();
     return cudaGetLastError();
 }
 
-cudaError_t qpi_forward_window(const void *holo, int bpc, int A, int N, int M, const int *carrier, float2 *T1,
-                               float2 *S, cudaStream_t s)
+cudaError_t qpi_forward_window(const float *bg, int nbg, const void *holo, int bpc, int A, int N, int M,
+                               const int *carrier, float2 *T1, float2 *S, cudaStream_t s)
 {
-    CTDM_DISPATCH_L(N, qpi_fwd_launch, holo, bpc, A, M, carrier, T1, S, s)
+    CTDM_DISPATCH_L(N, qpi_fwd_launch, bg, nbg, holo, bpc, A, M, carrier, T1, S, s)
 }
 
-cudaError_t qpi_inverse_window(float2 *S, int A, int M, const int *carrier, float2 *field_out, const float2 *bgf,
-                               long bg_stride, float *phase, float *amp, cudaStream_t s)
+cudaError_t qpi_inverse_rows(float2 *S, int A, int M, const int *carrier, cudaStream_t s)
 {
-    CTDM_DISPATCH_L(M, qpi_inv_launch, S, A, carrier, field_out, bgf, bg_stride, phase, amp, s)
+    CTDM_DISPATCH_L(M, qpi_inv_rows_launch, S, A, carrier, s)
+}
+
+cudaError_t qpi_inverse_cols(const float2 *S, int A, int M, const int *carrier, float2 *field_out, bool polar,
+                             const float2 *bgf, long bg_stride, float *phase, float *amp, cudaStream_t s)
+{
+    CTDM_DISPATCH_L(M, qpi_inv_cols_launch, S, A, carrier, field_out, polar, bgf, bg_stride, phase, amp, s)
 }
 
 // ------------------------------------------------------------ QPI Algorithm B
@@ -396,10 +448,13 @@ __device__ __forceinline__ float qpib_tap(const float *__restrict__ h, int N, fl
 }
 
 // holo: A holograms N x N; pairs q cover output rows (2q, 2q+1) of the A * N/4 rows.
+// Images: nbg of bg, then holograms of holo; image k's row pairs are the k-th N/8.
 // mag != NULL: |X| of the shifted spectrum rows (N floats per row).  Else T gets
-// the M = N/4 window columns per row, half-swapped.  center: device int.
+// the M = N/4 window columns per row, half-swapped, around center[1] for the first of holo's
+// images and center[0] for the others.
 template <int N>
-__global__ void __launch_bounds__(QRows<N>::THREADS) qpib_rows_kernel(const float *__restrict__ holo, long npairs,
+__global__ void __launch_bounds__(QRows<N>::THREADS) qpib_rows_kernel(const float *__restrict__ bg, int nbg,
+                                                                     const float *__restrict__ holo, long npairs,
                                                                      float *mag, float2 *T,
                                                                      const int *__restrict__ center,
                                                                      const float2 *__restrict__ tw)
@@ -413,14 +468,15 @@ __global__ void __launch_bounds__(QRows<N>::THREADS) qpib_rows_kernel(const floa
     const long q = (long)blockIdx.x * P::B + b;
     const bool ok = q < npairs;
     const long r0 = ok ? 2 * q : 0;                 // global output row (a * H + j)
-    const float *h0 = holo + (r0 / H) * (long)N * N, *h1 = holo + ((r0 + 1) / H) * (long)N * N;
-    const int j0 = (int)(r0 % H), j1 = (int)((r0 + 1) % H);
+    const int img = (int)(r0 / H);                  // H is even: both rows of one image
+    const float *h0 = img < nbg ? bg + (long)img * N * N : holo + (long)(img - nbg) * N * N;
+    const int j0 = (int)(r0 % H), j1 = j0 + 1;
     const float xr = (float)(N - 1) / (float)N, yr = (float)(N - 1) / (float)H;
     float2 v[P::E];
 #pragma unroll
     for (int i = 0; i < P::E; i++) {
         const int p = fftl::slot_pos<N, P::T, P::F0>(i, t);
-        v[i] = ok ? make_float2(qpib_tap(h0, N, xr, yr, p, j0), qpib_tap(h1, N, xr, yr, p, j1))
+        v[i] = ok ? make_float2(qpib_tap(h0, N, xr, yr, p, j0), qpib_tap(h0, N, xr, yr, p, j1))
                   : make_float2(0.f, 0.f);
     }
     P::template seq_row<false>(buf, v, tw);
@@ -440,7 +496,7 @@ __global__ void __launch_bounds__(QRows<N>::THREADS) qpib_rows_kernel(const floa
         }
         return;
     }
-    const int c = *center;
+    const int c = center[img == nbg ? 1 : 0];
     for (int x2 = t; x2 < M; x2 += P::T) {
         const int x = (x2 + M / 2) % M;             // half swap of the window
         const int ks = x - N / 8 + c;               // column of the shifted spectrum
@@ -456,16 +512,26 @@ __global__ void __launch_bounds__(QRows<N>::THREADS) qpib_rows_kernel(const floa
     }
 }
 
-// Column sums of |X| over the H rows of one hologram's spectrum, in row order, and
-// the first maximum over [int(0.6 N), N), mirrored to N - c when N - c < N/8.
-__global__ void qpib_center_kernel(const float *__restrict__ mag, int N, int H, int *center)
+// Column sums of |X| over the H rows of an image's spectrum, in row order, and the first
+// maximum over [int(0.6 N), N), mirrored to N - c when N - c < N/8.  CTA k: image k (the
+// background, then frame 1) into center[k]; the rows' loads go ahead of the ordered sum 32 at
+// a time.
+__global__ void __launch_bounds__(1024) qpib_center_kernel(const float *__restrict__ mag, int N, int H, int *center)
 {
     __shared__ unsigned long long best[32];
+    mag += (long)blockIdx.x * H * N;
     unsigned long long key = 0ull;
     const int lo = (int)(N * 0.6);
     for (int i = lo + threadIdx.x; i < N; i += blockDim.x) {
         float s = 0.f;
-        for (int j = 0; j < H; j++) s += mag[(long)j * N + i];
+        for (int j0 = 0; j0 < H; j0 += 32) {
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; j++) v[j] = j0 + j < H ? __ldg(&mag[(long)(j0 + j) * N + i]) : 0.f;
+#pragma unroll
+            for (int j = 0; j < 32; j++)
+                if (j0 + j < H) s += v[j];
+        }
         const unsigned long long k2 = ((unsigned long long)__float_as_uint(s) << 32) | (unsigned long long)(~(unsigned)i);
         if (k2 > key) key = k2;
     }
@@ -481,20 +547,28 @@ __global__ void qpib_center_kernel(const float *__restrict__ mag, int N, int H, 
             if (best[w] > k) k = best[w];
         int c = (int)(~(unsigned)(k & 0xffffffffull));
         if (N - c < (N / 4) / 2) c = N - c;
-        *center = c;
+        center[blockIdx.x] = c;
+        if (blockIdx.x == 0) center[2] = -1;   // Algorithm B has no radius
     }
 }
 
 // Inverse M-point transforms of the window rows, 1/M, conjugate, transposed store:
-// field[a][X * M + Y] from row Y, column X; with bgf the phase / amplitude epilogue
-// of calcWrapPhase instead (cTDM/HilbertTransform.cu:3618-3639).
+// field[a][X * M + Y] from row Y, column X (polar: as argument and modulus); with bgf the
+// phase / amplitude epilogue of calcWrapPhase instead (cTDM/HilbertTransform.cu:3618-3639).
+// 16 lines per CTA at M = 128 (twice the CTAs of the default plan): a scan of 49 frames of
+// 128 rows leaves a third of the SMs a second CTA of 32.
 template <int M>
-__global__ void __launch_bounds__(Plan<M>::THREADS) qpib_inv_kernel(const float2 *__restrict__ T, long nrows,
-                                                                   float2 *field_out, const float2 *__restrict__ bgf,
-                                                                   long bg_stride, float *phase, float *amp,
-                                                                   const float2 *__restrict__ tw)
+struct QbInv : Plan<M> {};
+template <> struct QbInv<128> : fftl::PlanT<128, 16, 8, fftl::Radices<16, 8>, fftl::Radices<8, 16>> {};
+
+template <int M>
+__global__ void __launch_bounds__(QbInv<M>::THREADS) qpib_inv_kernel(const float2 *__restrict__ T, long nrows,
+                                                                    float2 *field_out, bool polar,
+                                                                    const float2 *__restrict__ bgf, long bg_stride,
+                                                                    float *phase, float *amp,
+                                                                    const float2 *__restrict__ tw)
 {
-    using P = Plan<M>;
+    using P = QbInv<M>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
     const long row0 = (long)blockIdx.x * P::B;
@@ -515,53 +589,49 @@ __global__ void __launch_bounds__(Plan<M>::THREADS) qpib_inv_kernel(const float2
     const float sc = 1.0f / (float)M;
 #pragma unroll
     for (int i = 0; i < P::E; i++) {
-        const int X = fftl::slot_pos<M, P::T, P::RV0>(i, t);
+        const long o = (long)fftl::slot_pos<M, P::T, P::RV0>(i, t) * M + yy;
         const float2 f = make_float2(v[i].x * sc, -v[i].y * sc);
-        const long o = a * mm + (long)X * M + yy;
         if (field_out) {
-            field_out[o] = f;
+            field_out[a * mm + o] = polar ? to_polar(f) : f;
         } else {
-            const float2 g = bgf[a * bg_stride + (long)X * M + yy];
-            float ph = atan2f(g.y, g.x) - atan2f(f.y, f.x);
-            if (isnan(ph) || isinf(ph)) ph = 0.f;
-            float am = sqrtf(f.x * f.x + f.y * f.y) / sqrtf(g.x * g.x + g.y * g.y);
-            if (isnan(am) || isinf(am)) am = 0.f;
-            phase[o] = ph;
-            amp[o] = am;
+            float ph, am;
+            wrap_phase(f, bgf[a * bg_stride + o], ph, am);
+            phase[a * mm + o] = ph;
+            amp[a * mm + o] = am;
         }
     }
 }
 
 template <int N>
-static cudaError_t qpib_rows_launch(const float *holo, int A, float *mag, float2 *T, const int *center, cudaStream_t s)
+static cudaError_t qpib_rows_launch(const float *bg, int nbg, const float *holo, int A, float *mag, float2 *T,
+                                    const int *center, cudaStream_t s)
 {
     using PR = QRows<N>;
     if constexpr (N < 64) {
         return cudaErrorInvalidValue;
     } else {
         const size_t smem = fftl::plan_smem_row<PR>();
-        const long npairs = (long)A * (N / 4) / 2;
+        const long npairs = (long)(nbg + A) * (N / 4) / 2;
         cudaError_t e = set_smem<N>(qpib_rows_kernel<N>, smem);
         if (e != cudaSuccess) return e;
-        qpib_rows_kernel<N><<<(unsigned)((npairs + PR::B - 1) / PR::B), PR::THREADS, smem, s>>>(holo, npairs, mag, T,
-                                                                                              center, twiddles(N));
+        qpib_rows_kernel<N><<<(unsigned)((npairs + PR::B - 1) / PR::B), PR::THREADS, smem, s>>>(
+            bg, nbg, holo, npairs, mag, T, center, twiddles(N));
         note_launch();
         return cudaGetLastError();
     }
 }
 
 template <int M>
-static cudaError_t qpib_inv_launch(const float2 *T, int A, float2 *field_out, const float2 *bgf, long bg_stride,
-                                   float *phase, float *amp, cudaStream_t s)
+static cudaError_t qpib_inv_launch(const float2 *T, int A, float2 *field_out, bool polar, const float2 *bgf,
+                                   long bg_stride, float *phase, float *amp, cudaStream_t s)
 {
-    using P = Plan<M>;
-    const size_t smem = fftl::smem_bytes<M>();
+    using P = QbInv<M>;
+    const size_t smem = fftl::plan_smem<P>();
     cudaError_t e = set_smem<M>(qpib_inv_kernel<M>, smem);
     if (e != cudaSuccess) return e;
     const long nrows = (long)A * M;
-    qpib_inv_kernel<M><<<(unsigned)((nrows + P::B - 1) / P::B), P::THREADS, smem, s>>>(T, nrows, field_out, bgf,
-                                                                                      bg_stride, phase, amp,
-                                                                                      twiddles(M));
+    qpib_inv_kernel<M><<<(unsigned)((nrows + P::B - 1) / P::B), P::THREADS, smem, s>>>(
+        T, nrows, field_out, polar, bgf, bg_stride, phase, amp, twiddles(M));
     note_launch();
     return cudaGetLastError();
 }
@@ -598,8 +668,7 @@ __global__ void angcal_argmax_kernel(const float2 *__restrict__ spec, int N, lon
 cudaError_t angcal_peak(const float *img, int N, float2 *scratch, unsigned long long *key, cudaStream_t s)
 {
     const long n2 = (long)N * N;
-    real_to_complex_kernel<<<1024, 256, 0, s>>>(img, scratch, n2); note_launch();
-    cudaError_t e = fft_rows(scratch, N, N, false, s);
+    cudaError_t e = fft_rows_real(img, scratch, N, N, s);
     if (e == cudaSuccess) e = fft_cols(scratch, N, N, N, 0, N, false, s);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(key, 0, sizeof(unsigned long long), s);
@@ -608,33 +677,34 @@ cudaError_t angcal_peak(const float *img, int N, float2 *scratch, unsigned long 
     return cudaGetLastError();
 }
 
-cudaError_t qpib_spectrum_center(const float *holo, int N, float *mag, int *center, cudaStream_t s)
+cudaError_t qpib_centers(const float *bg, const float *frame1, int N, float *mag, int *center, cudaStream_t s)
 {
     cudaError_t e;
     switch (N) {
-    case 64: e = qpib_rows_launch<64>(holo, 1, mag, nullptr, nullptr, s); break;
-    case 128: e = qpib_rows_launch<128>(holo, 1, mag, nullptr, nullptr, s); break;
-    case 256: e = qpib_rows_launch<256>(holo, 1, mag, nullptr, nullptr, s); break;
-    case 512: e = qpib_rows_launch<512>(holo, 1, mag, nullptr, nullptr, s); break;
-    case 1024: e = qpib_rows_launch<1024>(holo, 1, mag, nullptr, nullptr, s); break;
-    case 2048: e = qpib_rows_launch<2048>(holo, 1, mag, nullptr, nullptr, s); break;
+    case 64: e = qpib_rows_launch<64>(bg, 1, frame1, 1, mag, nullptr, nullptr, s); break;
+    case 128: e = qpib_rows_launch<128>(bg, 1, frame1, 1, mag, nullptr, nullptr, s); break;
+    case 256: e = qpib_rows_launch<256>(bg, 1, frame1, 1, mag, nullptr, nullptr, s); break;
+    case 512: e = qpib_rows_launch<512>(bg, 1, frame1, 1, mag, nullptr, nullptr, s); break;
+    case 1024: e = qpib_rows_launch<1024>(bg, 1, frame1, 1, mag, nullptr, nullptr, s); break;
+    case 2048: e = qpib_rows_launch<2048>(bg, 1, frame1, 1, mag, nullptr, nullptr, s); break;
     default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
-    qpib_center_kernel<<<1, 1024, 0, s>>>(mag, N, N / 4, center);
+    qpib_center_kernel<<<2, 1024, 0, s>>>(mag, N, N / 4, center);
     note_launch();
     return cudaGetLastError();
 }
 
-cudaError_t qpib_window(const float *holo, int A, int N, const int *center, float2 *T, cudaStream_t s)
+cudaError_t qpib_window(const float *bg, int nbg, const float *holo, int A, int N, const int *center, float2 *T,
+                        cudaStream_t s)
 {
-    CTDM_DISPATCH_L(N, qpib_rows_launch, holo, A, nullptr, T, center, s)
+    CTDM_DISPATCH_L(N, qpib_rows_launch, bg, nbg, holo, A, nullptr, T, center, s)
 }
 
-cudaError_t qpib_inverse(const float2 *T, int A, int M, float2 *field_out, const float2 *bgf, long bg_stride,
-                         float *phase, float *amp, cudaStream_t s)
+cudaError_t qpib_inverse(const float2 *T, int A, int M, float2 *field_out, bool polar, const float2 *bgf,
+                         long bg_stride, float *phase, float *amp, cudaStream_t s)
 {
-    CTDM_DISPATCH_L(M, qpib_inv_launch, T, A, field_out, bgf, bg_stride, phase, amp, s)
+    CTDM_DISPATCH_L(M, qpib_inv_launch, T, A, field_out, polar, bgf, bg_stride, phase, amp, s)
 }
 
 }  // namespace ctdm

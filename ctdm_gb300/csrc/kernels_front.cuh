@@ -6,31 +6,37 @@ namespace ctdm {
 
 // QPI Algorithm A --------------------------------------------------------
 // Carrier of one background hologram (N x N float): carrier = {r, c, radius}
-// on the device.  scratch: N*N complex; key: one 64-bit word.
-cudaError_t qpi_find_carrier(const float *bg, int N, float2 *scratch, unsigned long long *key, int *carrier,
+// on the device.  scratch: N*N complex; state: two 64-bit words, zero before the call and
+// after it.
+cudaError_t qpi_find_carrier(const float *bg, int N, float2 *scratch, unsigned long long *state, int *carrier,
                              cudaStream_t s);
-// Pruned forward transform of A holograms into their M x M window spectra S
-// (ifftshifted, masked to the carrier's radius box: every entry of S is written, the
-// rows and columns outside the box with zeros).  T1: A*N*M complex scratch, of which
-// only the box's columns are used.
+// Pruned forward transform of nbg backgrounds (float) and A holograms into their M x M
+// window spectra S, the backgrounds' first (ifftshifted, masked to the carrier's radius box:
+// every entry of S is written, the rows and columns outside the box with zeros).
+// T1: (nbg + A)*N*M complex scratch, of which only the box's columns are used.
 // holo: A holograms of N x N pixels, bpc bytes each (4 float, 2 uint16, 1 uint8 counts)
-cudaError_t qpi_forward_window(const void *holo, int bpc, int A, int N, int M, const int *carrier, float2 *T1,
-                               float2 *S, cudaStream_t s);
-// Inverse M x M transform of an S written by qpi_forward_window with the same carrier
-// (destroyed; its zero rows are skipped) and the epilogue: field_out != NULL stores
-// the complex field, otherwise phase/amp against bgf[a * bg_stride].
-cudaError_t qpi_inverse_window(float2 *S, int A, int M, const int *carrier, float2 *field_out, const float2 *bgf,
-                               long bg_stride, float *phase, float *amp, cudaStream_t s);
+cudaError_t qpi_forward_window(const float *bg, int nbg, const void *holo, int bpc, int A, int N, int M,
+                               const int *carrier, float2 *T1, float2 *S, cudaStream_t s);
+// Inverse M x M transform of an S written by qpi_forward_window with the same carrier: the
+// rows in place (its zero rows are skipped), then the columns with the epilogue: field_out !=
+// NULL stores the complex field (polar: its argument and modulus), otherwise phase/amp
+// against the polar background bgf[a * bg_stride].
+cudaError_t qpi_inverse_rows(float2 *S, int A, int M, const int *carrier, cudaStream_t s);
+cudaError_t qpi_inverse_cols(const float2 *S, int A, int M, const int *carrier, float2 *field_out, bool polar,
+                             const float2 *bgf, long bg_stride, float *phase, float *amp, cudaStream_t s);
 
 // QPI Algorithm B --------------------------------------------------------
-// Carrier column of one hologram from its y-downsampled row spectra (mag: N/4 * N
-// floats of scratch; center: device int).
-cudaError_t qpib_spectrum_center(const float *holo, int N, float *mag, int *center, cudaStream_t s);
-// Window rows of A holograms (T: A * (N/4) rows of N/4 complex) for the carrier column.
-cudaError_t qpib_window(const float *holo, int A, int N, const int *center, float2 *T, cudaStream_t s);
-// Inverse window transforms into transposed fields, or phase/amp against bgf.
-cudaError_t qpib_inverse(const float2 *T, int A, int M, float2 *field_out, const float2 *bgf, long bg_stride,
-                         float *phase, float *amp, cudaStream_t s);
+// Carrier columns of the background (center[0]) and of frame 1 (center[1]) from their
+// y-downsampled row spectra (mag: 2 * N/4 * N floats of scratch; center: 3 device ints).
+cudaError_t qpib_centers(const float *bg, const float *frame1, int N, float *mag, int *center, cudaStream_t s);
+// Window rows (N/4 rows of N/4 complex per image) of nbg backgrounds, then of A holograms,
+// the first hologram's around center[1] and all others' around center[0].
+cudaError_t qpib_window(const float *bg, int nbg, const float *holo, int A, int N, const int *center, float2 *T,
+                        cudaStream_t s);
+// Inverse window transforms into transposed fields (polar: argument and modulus), or
+// phase/amp against the polar bgf.
+cudaError_t qpib_inverse(const float2 *T, int A, int M, float2 *field_out, bool polar, const float2 *bgf,
+                         long bg_stride, float *phase, float *amp, cudaStream_t s);
 
 // Angle camera: index of the spectrum peak of AngCal_GPU in *key's low word
 // (complemented; see angcal_peak).  scratch: N*N complex.
