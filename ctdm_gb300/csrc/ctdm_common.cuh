@@ -26,10 +26,10 @@ __device__ __forceinline__ float2 cmul_mi(float2 a)
     return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
-// The same pointer, opaque to the compiler: table loads through it stay where they are
-// written.  In a loop over line batches every thread's twiddles are loop-invariant, and
-// keeping them in registers across the loop (15 complex values per radix-16 stage) costs
-// more than reloading them from L1.
+// The same pointer, opaque to the compiler: loads through it stay behind this point (see
+// chain_begin), and in a loop over line batches, where every thread's twiddles are
+// loop-invariant, they are not kept in registers across it (15 complex values per radix-16
+// stage cost more than reloading them from L1).
 template <class T>
 __device__ __forceinline__ const T *fresh(const T *p)
 {

@@ -128,6 +128,8 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
                       const float2 *__restrict__ dtw, const float *__restrict__ eig, const float2 *__restrict__ tw)
 {
     namespace cg = cooperative_groups;
+    chain_begin();
+    phi = fresh(phi);
     using Y = fftl::Lay<M, P::LP, true>;
     constexpr int RPC = M / C, RL = 2 * P::B, E = P::E;
     static_assert(RPC % RL == 0 && P::T <= 32, "whole steps per CTA, a line within a warp");
@@ -297,13 +299,15 @@ static cudaError_t dct_phase(const float *phi, float *out, float *T, int A, int 
     cfg.blockDim = dim3(P::THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // chained (chain_begin)
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = C;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = PHASE == DCT_ALL ? 1 : 0;
+    cfg.numAttrs = PHASE == DCT_ALL ? 2 : 1;
     cudaError_t e = cudaLaunchKernelEx(&cfg, k, phi, T, out, mir, dtw, eig, tw);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();

@@ -42,6 +42,8 @@ static cudaError_t set_smem(K kernel, size_t smem)
 __global__ void __launch_bounds__(256) carrier_argmax_kernel(const float2 *__restrict__ spec, int N, int start,
                                                              unsigned long long *state, int *carrier)
 {
+    chain_begin();
+    spec = fresh(spec);
     unsigned long long best = 0ull;
     const long total = (long)(N - start) * N;
     for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
@@ -94,8 +96,7 @@ cudaError_t qpi_find_carrier(const float *bg, int N, float2 *scratch, unsigned l
     cudaError_t e = fft_rows_real(bg, scratch, N, N, s);
     if (e == cudaSuccess) e = fft_cols(scratch, N, N, N, 0, N, false, s);
     if (e != cudaSuccess) return e;
-    carrier_argmax_kernel<<<256, 256, 0, s>>>(scratch, N, (600 * N) / 1024, state, carrier); note_launch();
-    return cudaGetLastError();
+    return launch_chained(carrier_argmax_kernel, dim3(256), dim3(256), 0, s, scratch, N, (600 * N) / 1024, state, carrier);
 }
 
 // ------------------------------------------------------------ forward row pass
@@ -123,6 +124,10 @@ __global__ void __launch_bounds__(QRows<N>::THREADS, 1024 / QRows<N>::THREADS)
     qpi_rows_kernel(const float *__restrict__ bg, const T *__restrict__ holo, float2 *T1,
                     const int *__restrict__ carrier, long bgpairs, long npairs, int M, const float2 *__restrict__ tw)
 {
+    chain_begin();
+    bg = fresh(bg);
+    holo = fresh(holo);
+    carrier = fresh(carrier);
     using P = QRows<N>;
     using Y = fftl::Lay<N, P::LP, true>;
     extern __shared__ float4 smem4[];
@@ -194,6 +199,9 @@ __global__ void __launch_bounds__(QCols<N>::THREADS, 1024 / QCols<N>::THREADS)
     qpi_cols_kernel(const float2 *__restrict__ T1, float2 *S, const int *__restrict__ carrier, long nlines, int M,
                     const float2 *__restrict__ tw)
 {
+    chain_begin();
+    T1 = fresh(T1);
+    carrier = fresh(carrier);
     using P = QCols<N>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
@@ -248,6 +256,8 @@ __global__ void __launch_bounds__(Plan<M>::THREADS) qpi_rows_inv_kernel(float2 *
                                                                        const int *__restrict__ carrier,
                                                                        const float2 *__restrict__ tw)
 {
+    chain_begin();
+    carrier = fresh(carrier);
     using P = Plan<M>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
@@ -303,6 +313,10 @@ __global__ void __launch_bounds__(Plan<M>::THREADS) qpi_final_kernel(const float
                                                                     float *phase, float *amp,
                                                                     const float2 *__restrict__ tw)
 {
+    chain_begin();
+    S = fresh(S);
+    carrier = fresh(carrier);
+    bgf = fresh(bgf);
     using P = Plan<M>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
@@ -348,10 +362,8 @@ static cudaError_t qpi_rows_launch(const float *bg, int nbg, const T *holo, int 
     const long bgpairs = (long)nbg * N / 2, npairs = bgpairs + (long)A * N / 2;
     cudaError_t e = set_smem<N>(qpi_rows_kernel<N, T>, smem_r);
     if (e != cudaSuccess) return e;
-    qpi_rows_kernel<N, T><<<(unsigned)((npairs + PR::B - 1) / PR::B), PR::THREADS, smem_r, s>>>(
-        bg, holo, T1, carrier, bgpairs, npairs, M, twiddles(N));
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(qpi_rows_kernel<N, T>, dim3((unsigned)((npairs + PR::B - 1) / PR::B)), dim3(PR::THREADS),
+                          smem_r, s, bg, holo, T1, carrier, bgpairs, npairs, M, twiddles(N));
 }
 
 template <int N>
@@ -368,9 +380,8 @@ static cudaError_t qpi_fwd_launch(const float *bg, int nbg, const void *holo, in
     const size_t smem = fftl::plan_smem<PC>();
     e = set_smem<N>(qpi_cols_kernel<N>, smem);
     if (e != cudaSuccess) return e;
-    qpi_cols_kernel<N><<<(unsigned)((nl + PC::B - 1) / PC::B), PC::THREADS, smem, s>>>(T1, S, carrier, nl, M,
-                                                                                      twiddles(N)); note_launch();
-    return cudaGetLastError();
+    return launch_chained(qpi_cols_kernel<N>, dim3((unsigned)((nl + PC::B - 1) / PC::B)), dim3(PC::THREADS), smem, s,
+                          T1, S, carrier, nl, M, twiddles(N));
 }
 
 template <int M>
@@ -381,9 +392,8 @@ static cudaError_t qpi_inv_rows_launch(float2 *S, int A, const int *carrier, cud
     const size_t smem_r = fftl::plan_smem_row<P>();
     cudaError_t e = set_smem<M>(qpi_rows_inv_kernel<M>, smem_r);
     if (e != cudaSuccess) return e;
-    qpi_rows_inv_kernel<M><<<(unsigned)((nl + P::B - 1) / P::B), P::THREADS, smem_r, s>>>(S, nl, carrier,
-                                                                                         twiddles(M)); note_launch();
-    return cudaGetLastError();
+    return launch_chained(qpi_rows_inv_kernel<M>, dim3((unsigned)((nl + P::B - 1) / P::B)), dim3(P::THREADS), smem_r, s,
+                          S, nl, carrier, twiddles(M));
 }
 
 template <int M>
@@ -395,10 +405,8 @@ static cudaError_t qpi_inv_cols_launch(const float2 *S, int A, const int *carrie
     const size_t smem = fftl::smem_bytes<M>();
     cudaError_t e = set_smem<M>(qpi_final_kernel<M>, smem);
     if (e != cudaSuccess) return e;
-    qpi_final_kernel<M><<<(unsigned)((nl + P::B - 1) / P::B), P::THREADS, smem, s>>>(
-        S, nl, carrier, field_out, polar, bgf, bg_stride, phase, amp, twiddles(M));
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(qpi_final_kernel<M>, dim3((unsigned)((nl + P::B - 1) / P::B)), dim3(P::THREADS), smem, s, S,
+                          nl, carrier, field_out, polar, bgf, bg_stride, phase, amp, twiddles(M));
 }
 
 cudaError_t qpi_forward_window(const float *bg, int nbg, const void *holo, int bpc, int A, int N, int M,
@@ -459,6 +467,10 @@ __global__ void __launch_bounds__(QRows<N>::THREADS) qpib_rows_kernel(const floa
                                                                      const int *__restrict__ center,
                                                                      const float2 *__restrict__ tw)
 {
+    chain_begin();
+    bg = fresh(bg);
+    holo = fresh(holo);
+    center = fresh(center);
     using P = QRows<N>;
     using Y = fftl::Lay<N, P::LP, true>;
     constexpr int H = N / 4, M = N / 4;
@@ -514,26 +526,32 @@ __global__ void __launch_bounds__(QRows<N>::THREADS) qpib_rows_kernel(const floa
 
 // Column sums of |X| over the H rows of an image's spectrum, in row order, and the first
 // maximum over [int(0.6 N), N), mirrored to N - c when N - c < N/8.  CTA k: image k (the
-// background, then frame 1) into center[k]; the rows' loads go ahead of the ordered sum 32 at
-// a time.
+// background, then frame 1) into center[k].  Blocks of rows are staged in shared memory by
+// all threads; the ordered sums then run from there, one thread per column.
+constexpr int QB_STAGE = 24 * 1024;   // floats
 __global__ void __launch_bounds__(1024) qpib_center_kernel(const float *__restrict__ mag, int N, int H, int *center)
 {
+    chain_begin();
+    mag = fresh(mag);
+    extern __shared__ float srow[];
     __shared__ unsigned long long best[32];
     mag += (long)blockIdx.x * H * N;
-    unsigned long long key = 0ull;
-    const int lo = (int)(N * 0.6);
-    for (int i = lo + threadIdx.x; i < N; i += blockDim.x) {
-        float s = 0.f;
-        for (int j0 = 0; j0 < H; j0 += 32) {
-            float v[32];
-#pragma unroll
-            for (int j = 0; j < 32; j++) v[j] = j0 + j < H ? __ldg(&mag[(long)(j0 + j) * N + i]) : 0.f;
-#pragma unroll
-            for (int j = 0; j < 32; j++)
-                if (j0 + j < H) s += v[j];
+    const int lo = (int)(N * 0.6), nc = N - lo, step = min(H, QB_STAGE / nc);
+    float s = 0.f;   // nc <= 820 columns: at most one per thread
+    for (int j0 = 0; j0 < H; j0 += step) {
+        const int rows = min(step, H - j0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < rows * nc; e += 1024) srow[e] = __ldg(&mag[(long)(j0 + e / nc) * N + lo + e % nc]);
+        __syncthreads();
+        if ((int)threadIdx.x < nc) {
+#pragma unroll 8
+            for (int j = 0; j < rows; j++) s += srow[j * nc + threadIdx.x];
         }
-        const unsigned long long k2 = ((unsigned long long)__float_as_uint(s) << 32) | (unsigned long long)(~(unsigned)i);
-        if (k2 > key) key = k2;
+    }
+    unsigned long long key = 0ull;
+    if ((int)threadIdx.x < nc) {
+        const unsigned i = lo + threadIdx.x;
+        key = ((unsigned long long)__float_as_uint(s) << 32) | (unsigned long long)(~i);
     }
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long other = __shfl_xor_sync(0xffffffffu, key, o);
@@ -543,7 +561,7 @@ __global__ void __launch_bounds__(1024) qpib_center_kernel(const float *__restri
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long k = best[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++)
+        for (int w = 1; w < 32; w++)
             if (best[w] > k) k = best[w];
         int c = (int)(~(unsigned)(k & 0xffffffffull));
         if (N - c < (N / 4) / 2) c = N - c;
@@ -568,6 +586,9 @@ __global__ void __launch_bounds__(QbInv<M>::THREADS) qpib_inv_kernel(const float
                                                                     float *phase, float *amp,
                                                                     const float2 *__restrict__ tw)
 {
+    chain_begin();
+    T = fresh(T);
+    bgf = fresh(bgf);
     using P = QbInv<M>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
@@ -614,10 +635,8 @@ static cudaError_t qpib_rows_launch(const float *bg, int nbg, const float *holo,
         const long npairs = (long)(nbg + A) * (N / 4) / 2;
         cudaError_t e = set_smem<N>(qpib_rows_kernel<N>, smem);
         if (e != cudaSuccess) return e;
-        qpib_rows_kernel<N><<<(unsigned)((npairs + PR::B - 1) / PR::B), PR::THREADS, smem, s>>>(
-            bg, nbg, holo, npairs, mag, T, center, twiddles(N));
-        note_launch();
-        return cudaGetLastError();
+        return launch_chained(qpib_rows_kernel<N>, dim3((unsigned)((npairs + PR::B - 1) / PR::B)), dim3(PR::THREADS),
+                              smem, s, bg, nbg, holo, npairs, mag, T, center, twiddles(N));
     }
 }
 
@@ -630,10 +649,8 @@ static cudaError_t qpib_inv_launch(const float2 *T, int A, float2 *field_out, bo
     cudaError_t e = set_smem<M>(qpib_inv_kernel<M>, smem);
     if (e != cudaSuccess) return e;
     const long nrows = (long)A * M;
-    qpib_inv_kernel<M><<<(unsigned)((nrows + P::B - 1) / P::B), P::THREADS, smem, s>>>(
-        T, nrows, field_out, polar, bgf, bg_stride, phase, amp, twiddles(M));
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(qpib_inv_kernel<M>, dim3((unsigned)((nrows + P::B - 1) / P::B)), dim3(P::THREADS), smem, s, T,
+                          nrows, field_out, polar, bgf, bg_stride, phase, amp, twiddles(M));
 }
 
 // ------------------------------------------------------------ angle camera (AngCal_GPU)
@@ -690,9 +707,10 @@ cudaError_t qpib_centers(const float *bg, const float *frame1, int N, float *mag
     default: return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
-    qpib_center_kernel<<<2, 1024, 0, s>>>(mag, N, N / 4, center);
-    note_launch();
-    return cudaGetLastError();
+    const size_t smem = sizeof(float) * QB_STAGE;
+    if ((e = cudaFuncSetAttribute(qpib_center_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+        return e;
+    return launch_chained(qpib_center_kernel, dim3(2), dim3(1024), smem, s, mag, N, N / 4, center);
 }
 
 cudaError_t qpib_window(const float *bg, int nbg, const float *holo, int A, int N, const int *center, float2 *T,

@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(ColPlan<L>::THREADS) cols_kernel(const float2 
                                                                    long plane, long ld, float scale,
                                                                    const int *__restrict__ xactive)
 {
+    chain_begin();
+    xactive = fresh(xactive);
     using P = ColPlan<L>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
@@ -142,8 +144,8 @@ static cudaError_t cols_launch(const float2 *src, float2 *data, long nlines, int
     auto k = inv ? cols_kernel<L, true> : cols_kernel<L, false>;
     cudaError_t e = prep_launch<L>(k, smem);
     if (e != cudaSuccess) return e;
-    k<<<(unsigned)grid, P::THREADS, smem, s>>>(src, data, twiddles(L), nlines, nx, plane, ld, scale, xactive); note_launch();
-    return cudaGetLastError();
+    return launch_chained(k, dim3((unsigned)grid), dim3(P::THREADS), smem, s, src, data, twiddles(L), nlines, nx, plane, ld,
+                          scale, xactive);
 }
 
 cudaError_t fft_rows(float2 *data, int L, long nlines, bool inverse, cudaStream_t s)
@@ -297,6 +299,7 @@ template <class P, bool FI, bool ZINV>
 __global__ void __launch_bounds__(EwaldCfg<P, ZINV>::THREADS)
     ewald_kernel(EwaldArgs a, EwaldRange rg, unsigned body, const float2 *__restrict__ tw)
 {
+    chain_begin();
     constexpr int R = P::L, B = EwaldCfg<P, ZINV>::B, THREADS = EwaldCfg<P, ZINV>::THREADS;
     extern __shared__ float4 smem4[];
     float2 *acc = reinterpret_cast<float2 *>(smem4);                    // [plane][column]
@@ -412,9 +415,8 @@ static cudaError_t ewald_run(const EwaldArgs &a, cudaStream_t s)
     cudaError_t e = prep_launch<L>(k, smem);
     if (e != cudaSuccess) return e;
     using Cfg = EwaldCfg<P, ZINV>;
-    k<<<(unsigned)((long)L * L / Cfg::B), Cfg::THREADS, smem, s>>>(a, rg, body, twiddles(L));
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(k, dim3((unsigned)((long)L * L / Cfg::B)), dim3(Cfg::THREADS), smem, s, a, rg, body,
+                          twiddles(L));
 }
 
 template <int L>
@@ -434,6 +436,9 @@ __global__ void __launch_bounds__(256) pack_measured_kernel(const float2 *__rest
                                                            int *tcount, int *tprefix, float2 *tvals, int *active,
                                                            PackRule rule)
 {
+    chain_begin();
+    F2 = fresh(F2);
+    mask = fresh(mask);
     extern __shared__ int spre[];   // R prefixes, then 8 warp totals
     int *swarp = spre + R;
     constexpr int ZR = 256 / TB;    // z rows per step
@@ -519,14 +524,9 @@ cudaError_t pack_measured(const float2 *F2, const uint8_t *mask, int R, int TB, 
     if (R > 768) return cudaErrorInvalidValue;
     const unsigned tiles = (unsigned)((long)R * R / TB);
     const size_t smem = sizeof(int) * (R + 8);
-    switch (TB) {
-    case 8: pack_measured_kernel<8><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active, rule); break;
-    case 16: pack_measured_kernel<16><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active, rule); break;
-    case 32: pack_measured_kernel<32><<<tiles, 256, smem, s>>>(F2, mask, R, tmask, tcount, tprefix, tvals, active, rule); break;
-    default: return cudaErrorInvalidValue;
-    }
-    note_launch();
-    return cudaGetLastError();
+    auto k = TB == 8 ? pack_measured_kernel<8> : (TB == 16 ? pack_measured_kernel<16> : pack_measured_kernel<32>);
+    if (TB != 8 && TB != 16 && TB != 32) return cudaErrorInvalidValue;
+    return launch_chained(k, dim3(tiles), dim3(256), smem, s, F2, mask, R, tmask, tcount, tprefix, tvals, active, rule);
 }
 
 // Volume sides supported by the reconstruction passes.

@@ -270,6 +270,9 @@ __global__ void __launch_bounds__(256) prep_resize_kernel(const float *__restric
                                                          const float *__restrict__ amp, int M, int N, int R,
                                                          float2 *U0)
 {
+    chain_begin();
+    phase = fresh(phase);
+    amp = fresh(amp);
     __shared__ float hp[PR_ROWS][PR_LD], ha[PR_ROWS][PR_LD];
     const int map = blockIdx.z, tx0 = blockIdx.x * PR_X, ty0 = blockIdx.y * PR_Y;
     const float *P = phase + (long)map * M * M, *Am = amp + (long)map * M * M;
@@ -358,7 +361,7 @@ cudaError_t prep_rytov(const float *phase, const float *amp, int A, int M, int N
     const dim3 block(32, 8);
     if (M - 1 <= N) {
         const dim3 grid((R + PR_X - 1) / PR_X, (R + PR_Y - 1) / PR_Y, A);
-        prep_resize_kernel<<<grid, block, 0, s>>>(phase, amp, M, N, R, U0);
+        return launch_chained(prep_resize_kernel, grid, block, 0, s, phase, amp, M, N, R, U0);
     } else {
         const dim3 grid((R + 31) / 32, (R + 31) / 32, A);
         prep_kernel<0, 0><<<grid, block, 0, s>>>(phase, amp, M, N, R, U0, nullptr, nullptr);

@@ -20,6 +20,37 @@ const float2 *twiddles(int L);
 const float2 *dct_twiddles(int M);
 const float *dct_eigen(int M);
 
+// ---- chained launches
+// A kernel that starts with chain_begin() may be launched with launch_chained: its CTAs are
+// then scheduled while the last ones of the kernel before it in the stream still run, and
+// wait in chain_begin until that kernel has completed and its writes are visible, so that
+// the launch latency is hidden.  Nothing but the tables is read or written before
+// chain_begin, and const __restrict__ inputs go through fresh() after it, so that the
+// compiler cannot take their loads for invariant and move them ahead.  (Every
+// kernel of a chain waits for the one before it, so the wait covers all earlier ones.)
+__device__ __forceinline__ void chain_begin()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... KA, class... A>
+cudaError_t launch_chained(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
+    note_launch();
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 // ---- per-angle Ewald geometry (host computed, FP64 rule inputs)
 struct AngleGeom {
     double fx0, fy0, fz0;  // illumination frequency (1/m); fx0 = fm0 sin(AngY), fy0 = fm0 sin(AngX)

@@ -34,6 +34,7 @@ template <class P, bool INV, class LD, class ST>
 __global__ void __launch_bounds__(P::THREADS, row_min_ctas<P>())
     rows_fn_kernel(LD ld, ST st, const float2 *__restrict__ tw, long nlines)
 {
+    chain_begin();
     constexpr int L = P::L;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
@@ -114,9 +115,8 @@ static cudaError_t rows_fn_launch(LD ld, ST st, long nlines, cudaStream_t s)
     auto k = rows_fn_kernel<P, INV, LD, ST>;
     const cudaError_t e = prep_line_kernel(reinterpret_cast<const void *>(k), P::L, smem);
     if (e != cudaSuccess) return e;
-    k<<<(unsigned)((nlines + P::B - 1) / P::B), P::THREADS, smem, s>>>(ld, st, twiddles(P::L), nlines);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(k, dim3((unsigned)((nlines + P::B - 1) / P::B)), dim3(P::THREADS), smem, s, ld, st,
+                          twiddles(P::L), nlines);
 }
 
 struct LoadComplex {

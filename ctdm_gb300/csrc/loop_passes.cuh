@@ -43,6 +43,11 @@ static cudaError_t prep_plan_kernel(K kernel, int L, size_t smem)
     return e;
 }
 
+// Sides whose passes are launched chained: at 64^3 a pass takes 3 to 4 us and the gap to the
+// next one another 1.3; five loop bodies with the chained front end went from 248 to 202 us
+// (16 x 256^2 frames -> 64^3).  At 256^3 a pass hides nothing that shows.
+constexpr bool chain_passes(int L) { return L <= 128; }
+
 // Lines one wave ahead for a z-pass kernel: its resident CTAs on the device x lines per
 // CTA (0 when the occupancy query fails), once per kernel and device.  A z-pass CTA
 // prefetches into L2 the z lines of the CTA that starts when it ends, so that CTA's
@@ -92,6 +97,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4)) xpass_k
                                                                                       const float2 *__restrict__ tw)
 {
     constexpr int L = P::L;
+    if constexpr (chain_passes(L)) chain_begin();
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
     const int t = threadIdx.x % P::T, b = threadIdx.x / P::T;
@@ -145,6 +151,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(5)) ypass_k
                                                                                       const float2 *__restrict__ tw)
 {
     constexpr int L = P::L;
+    if constexpr (chain_passes(L)) chain_begin();
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
     // planes in descending z: the x pass runs them ascending, so each pass starts on
@@ -199,6 +206,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(3))
     constexpr int L = P::L;
     constexpr bool TMA = zpass_tma<P>();
     const bool staged = TMA && a.staged;   // uniform over the grid
+    if constexpr (chain_passes(L)) chain_begin();
     extern __shared__ float4 smem4[];
     // [F2 tile, z-major: B*L float2][mask tile B*L bytes][FFT buffer][mbarrier], 128-byte aligned
     char *base0 = reinterpret_cast<char *>(smem4);
@@ -292,6 +300,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4))
     zpass_packed_kernel(LoopArgs a, const float2 *__restrict__ tw, int ahead)
 {
     constexpr int L = P::L;
+    if constexpr (chain_passes(L)) chain_begin();
     extern __shared__ float4 smem4[];
     char *base0 = reinterpret_cast<char *>(smem4);
     char *al = base0 + ((128 - (tma::smem_addr(base0) & 127)) & 127);
@@ -347,6 +356,18 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4))
 
 // ------------------------------------------------------------ launchers
 // kind: LOOP_X, LOOP_X_FINAL, LOOP_Y_FWD, LOOP_Y_INV, LOOP_Z (flag = check mode)
+template <int L, class K, class... A>
+static cudaError_t launch_pass(K k, unsigned grid, int threads, size_t smem, cudaStream_t s, A... args)
+{
+    if constexpr (chain_passes(L)) {
+        return launch_chained(k, dim3(grid), dim3(threads), smem, s, args...);
+    } else {
+        k<<<grid, threads, smem, s>>>(args...);
+        note_launch();
+        return cudaGetLastError();
+    }
+}
+
 template <class P>
 static cudaError_t run_loop_pass(int kind, const LoopArgs &a, int flag, cudaStream_t s)
 {
@@ -359,19 +380,19 @@ static cudaError_t run_loop_pass(int kind, const LoopArgs &a, int flag, cudaStre
                                       : (a.xprev ? xpass_kernel<P, false, true> : xpass_kernel<P, false>);
         e = prep_plan_kernel(k, L, smem);
         if (e != cudaSuccess) return e;
-        k<<<grid, P::THREADS, smem, s>>>(a, twiddles(L));
+        return launch_pass<L>(k, grid, P::THREADS, smem, s, a, twiddles(L));
     } else if (kind == LOOP_Y_FWD || kind == LOOP_Y_INV) {
         const size_t smem = fftl::plan_smem<P>();
         auto k = kind == LOOP_Y_INV ? ypass_kernel<P, true> : ypass_kernel<P, false>;
         e = prep_plan_kernel(k, L, smem);
         if (e != cudaSuccess) return e;
-        k<<<grid, P::THREADS, smem, s>>>(a, twiddles(L));
+        return launch_pass<L>(k, grid, P::THREADS, smem, s, a, twiddles(L));
     } else if (a.packed && zpass_packable<P>()) {
         const size_t smem = zpass_packed_smem<P>();
         auto k = zpass_packed_kernel<P>;
         e = prep_plan_kernel(k, L, smem);
         if (e != cudaSuccess) return e;
-        k<<<grid, P::THREADS, smem, s>>>(a, twiddles(L), (int)(zpass_ahead<P>(k, smem) / P::B));
+        return launch_pass<L>(k, grid, P::THREADS, smem, s, a, twiddles(L), (int)(zpass_ahead<P>(k, smem) / P::B));
     } else {
         const size_t smem = flag ? zpass_smem<P, 1>() : zpass_smem<P, 0>();
         auto k = flag ? zpass_kernel<P, 1> : zpass_kernel<P, 0>;
@@ -390,10 +411,8 @@ static cudaError_t run_loop_pass(int kind, const LoopArgs &a, int flag, cudaStre
             if (okmap && flag) okmap = tma::make_map_3d(&maskmap, a.mask, 1, dims, box) == cudaSuccess;
             la.staged = okmap ? 1 : 0;
         }
-        k<<<grid, P::THREADS, smem, s>>>(la, twiddles(L), f2map, maskmap, zpass_ahead<P>(k, smem));
+        return launch_pass<L>(k, grid, P::THREADS, smem, s, la, twiddles(L), f2map, maskmap, zpass_ahead<P>(k, smem));
     }
-    note_launch();
-    return cudaGetLastError();
 }
 
 // Lines per z-pass CTA when that plan reads packed measured samples, else 0.
