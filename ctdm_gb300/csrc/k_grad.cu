@@ -240,6 +240,7 @@ template <class P, int MODE>
 __global__ void __launch_bounds__(P::THREADS, P::E <= 16 ? 1024 / P::THREADS : 512 / P::THREADS)
     tape_z_kernel(TapeZ a, const float2 *__restrict__ tw)
 {
+    chain_begin();
     constexpr bool RES = MODE == Z_RESIDUAL || MODE == Z_RESIDUAL_SUM;
     constexpr int L = P::L;
     static_assert(P::B <= 32 && P::B <= L, "one mask word per z row of a tile");
@@ -315,9 +316,7 @@ static cudaError_t tape_z_launch(TapeZ a, cudaStream_t s)
     cudaError_t e = prep_line_kernel(reinterpret_cast<const void *>(k), L, smem);
     if (e != cudaSuccess) return e;
     a.ahead = wave_ctas(k, P::THREADS, smem);
-    k<<<(unsigned)((long)L * L / P::B), P::THREADS, smem, s>>>(a, twiddles(L));
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(k, dim3((unsigned)((long)L * L / P::B)), dim3(P::THREADS), smem, s, a, twiddles(L));
 }
 
 #define CTDM_SIDES(FN, ...)                                 \
@@ -420,6 +419,7 @@ __device__ __forceinline__ float tv_inv(float2 dx, float2 dy, float2 dz, float e
 template <bool UPDATE>
 __global__ void __launch_bounds__(kTvThreads, 3) tv_kernel(TvArgs a)
 {
+    chain_begin();
     __shared__ float2 pl[2][kTvH][kTvW];           // planes z and z + 1, one-voxel halo
     __shared__ float2 qx[kTvY][kTvX + 1], qy[kTvY + 1][kTvX];   // q of the tile and its x / y halo
     const int R = a.R, nbx = R / kTvX, nby = R / kTvY;
@@ -544,9 +544,7 @@ template <bool UPDATE>
 cudaError_t launch_tv(TvArgs a, cudaStream_t s)
 {
     a.zc = tv_planes<UPDATE>(a.R);
-    tv_kernel<UPDATE><<<tv_grid<UPDATE>(a.R), kTvThreads, 0, s>>>(a);
-    note_launch();
-    return cudaGetLastError();
+    return launch_chained(tv_kernel<UPDATE>, dim3(tv_grid<UPDATE>(a.R)), dim3(kTvThreads), 0, s, a);
 }
 
 // n = n_med sqrt(1 + V) (principal root), optional positivity clamp, octant shift.
