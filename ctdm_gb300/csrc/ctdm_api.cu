@@ -926,7 +926,8 @@ static ctdm_status pipeline_core(ctdm_ctx *c, const ctdm_params *p, int A, int M
     auto goldstein_all = [&](cudaStream_t gs) -> ctdm_status {
         const float *ph_all = B<float>(c, B_PHASE);
         CK(goldstein_residues(ph_all, A, M, M, B<int8_t>(c, B_CHG), gs), "goldstein residues");
-        CK(goldstein_cuts(B<int8_t>(c, B_CHG), A, M, M, B<uint8_t>(c, B_CUT), B<int8_t>(c, B_GWORK), gs),
+        CK(goldstein_cuts(B<int8_t>(c, B_CHG), A, M, M, B<uint8_t>(c, B_CUT), B<int8_t>(c, B_GWORK),
+                          !gold_feeds, gs),
            "goldstein cuts");
         CK(goldstein_floodfill(B<uint8_t>(c, B_CUT), ph_all, A, M, M, B<float>(c, B_GOLD), B<uint8_t>(c, B_GSTATE),
                                B<int>(c, B_GLIST), B<int>(c, B_GSTATUS), gs),
@@ -1353,7 +1354,7 @@ extern "C" ctdm_status ctdm_goldstein(ctdm_ctx *c, int A, int W, int H, const fl
     CK(ensure(c, B_GSTATUS, sizeof(int) * A), "alloc status");
     CK(ensure(c, B_TMP, A * n), "alloc work");
     CK(goldstein_residues(d_phi, A, W, H, d_charges, s), "residues");
-    CK(goldstein_cuts(d_charges, A, W, H, d_cuts, B<int8_t>(c, B_TMP), s), "branch cuts");
+    CK(goldstein_cuts(d_charges, A, W, H, d_cuts, B<int8_t>(c, B_TMP), false, s), "branch cuts");
     CK(goldstein_floodfill(d_cuts, d_phi, A, W, H, d_out, B<uint8_t>(c, B_GSTATE), B<int>(c, B_GLIST),
                            B<int>(c, B_GSTATUS), s),
        "flood fill");

@@ -125,46 +125,67 @@ __device__ __forceinline__ void seq_cell(unsigned s, unsigned m1, unsigned m2, u
     nn = n1 + s;
 }
 
-// Residues of a map in index order, gathered before any cut is placed: lanes load
-// CUTS_BATCH bytes each per step, all independent (the charges are mostly zero, and
-// one dependent load per 32 pixels made the scan most of the kernel's time).  Pairing
-// only clears charges, so a gathered residue that is already paired is skipped.
-constexpr int CUTS_BATCH = 32, CUTS_LIST = 2048;
+// Residues of a map in index order, gathered before any cut is placed by WARPS warps (the map
+// in as many spans; the spans' counts give each its place in the list): 16 independent bytes
+// per lane in flight.  Pairing only clears charges, so a gathered residue that is already
+// paired is skipped.  One warp then walks the list: its order is the specification.
+//   WARPS = 8 where the caller waits for the cuts: 49 maps of 256^2 in 24 us, 87 us with one
+//   warp (the latency of the gather).
+//   WARPS = 1 beside the loop (side stream), where nothing waits: the 8-warp CTAs, and the
+//   fill that they let start 60 us earlier, take SMs while the plane pass's clusters are
+//   being placed.  49 angles at 256^3 with the loop: 4.42 ms with one warp, 4.65 with 8.
+constexpr int CUTS_BATCH = 16, CUTS_LIST = 2048, CUTS_WARPS = 8;
 
-__global__ void __launch_bounds__(32) cuts_kernel(const int8_t *__restrict__ charges, int W, int H, uint8_t *cuts,
-                                                  int8_t *work)
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) cuts_kernel(const int8_t *__restrict__ charges, int W, int H,
+                                                          uint8_t *cuts, int8_t *work)
 {
     __shared__ unsigned s_res[CUTS_LIST];
-    const int a = blockIdx.x, lane = threadIdx.x;
+    __shared__ int s_cnt[WARPS];
+    const int a = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long n = (long)W * H;
     volatile int8_t *masked = work + a * n;
     volatile uint8_t *cut = cuts + a * n;
     const int8_t *__restrict__ q = charges + a * n;
-    int nres = 0;
-    for (long base = 0; base < n; base += 32 * CUTS_BATCH) {
-        int v[CUTS_BATCH];
+    const long span = (n + WARPS - 1) / WARPS, p0 = warp * span, p1 = min(n, p0 + span);
+    int at = 0;   // pass 0 counts the span's residues, pass 1 lists them from their place on
+    constexpr int LIST = WARPS > 1;   // one warp: one pass does both
+    for (int pass = 0; pass <= LIST; pass++) {
+        for (long base = p0; base < p1; base += 32 * CUTS_BATCH) {
+            int v[CUTS_BATCH];
 #pragma unroll
-        for (int k = 0; k < CUTS_BATCH; k++) {
-            const long pl = base + 32 * k + lane;
-            v[k] = pl < n ? __ldg(q + pl) : 0;
+            for (int k = 0; k < CUTS_BATCH; k++) {
+                const long pl = base + 32 * k + lane;
+                v[k] = pl < p1 ? __ldg(q + pl) : 0;
+            }
+#pragma unroll
+            for (int k = 0; k < CUTS_BATCH; k++) {
+                const long pl = base + 32 * k + lane;
+                const unsigned hit = __ballot_sync(0xffffffffu, v[k] != 0);
+                if (pass == 0) {
+                    if (pl < p1) {
+                        masked[pl] = (int8_t)v[k];
+                        cut[pl] = 0;
+                    }
+                }
+                if (pass == LIST && v[k] != 0) {
+                    const int i = at + __popc(hit & ((1u << lane) - 1u));
+                    if (i < CUTS_LIST) s_res[i] = (unsigned)pl;
+                }
+                at += __popc(hit);
+            }
         }
-#pragma unroll
-        for (int k = 0; k < CUTS_BATCH; k++) {
-            const long pl = base + 32 * k + lane;
-            if (pl < n) {
-                masked[pl] = (int8_t)v[k];
-                cut[pl] = 0;
-            }
-            unsigned pend = __ballot_sync(0xffffffffu, v[k] != 0);
-            while (pend) {
-                const int l = __ffs(pend) - 1;
-                pend &= pend - 1;
-                if (lane == 0 && nres < CUTS_LIST) s_res[nres] = (unsigned)(base + 32 * k + l);
-                nres++;
-            }
+        if (pass == 0) {
+            if (lane == 0) s_cnt[warp] = at;
+            __syncthreads();
+            if (LIST) at = 0;
+            for (int w = 0; w < warp; w++) at += s_cnt[w];
         }
     }
-    __syncwarp();
+    __syncthreads();
+    if (warp != 0) return;
+    int nres = 0;
+    for (int w = 0; w < WARPS; w++) nres += s_cnt[w];
     int maxBox = 901;
     const int half = (int)floorf((float)(W / 2));
     if (half < maxBox) maxBox = half;
@@ -256,9 +277,14 @@ __global__ void __launch_bounds__(32) cuts_kernel(const int8_t *__restrict__ cha
     }
 }
 
-cudaError_t goldstein_cuts(const int8_t *charges, int A, int W, int H, uint8_t *cuts, int8_t *work, cudaStream_t s)
+cudaError_t goldstein_cuts(const int8_t *charges, int A, int W, int H, uint8_t *cuts, int8_t *work, bool beside,
+                           cudaStream_t s)
 {
-    cuts_kernel<<<A, 32, 0, s>>>(charges, W, H, cuts, work); note_launch();
+    if (beside)
+        cuts_kernel<1><<<A, 32, 0, s>>>(charges, W, H, cuts, work);
+    else
+        cuts_kernel<CUTS_WARPS><<<A, 32 * CUTS_WARPS, 0, s>>>(charges, W, H, cuts, work);
+    note_launch();
     return cudaGetLastError();
 }
 
@@ -479,17 +505,20 @@ __device__ void sweep(uint8_t *st, const FFLists &ls, int L, int *nnext, const f
 //   1. conversion, candidates (from UB and CUT, which no phase of the sweep changes),
 //      loads of ph[p] and of the neighbours' old values in o;
 //   2. F_PREV cleared on the previous list's pixels outside this list (the owners
-//      clear their own), and the fixed point over left / upper neighbours;
+//      clear their own), and, only when some pixel has no unwrapped neighbour yet (*s_fix),
+//      the fixed point over left / upper neighbours;
 //   3. reference neighbour; a value whose reference is not a pixel of this sweep
 //      computed from the loaded old value and stored in o at once (every read of an
 //      old value was issued before barrier 1);
-//   4. dependency rounds, only when some pixel waits on another of this sweep;
+//   4. dependency rounds, only when some pixel waits on another of this sweep: a value is
+//      published (value, fence, F_READY) as soon as its reference is, so a round may take
+//      several steps of a chain;
 //   5. adjoin marks (atomics only); 6. the final states.
 // Plain stores to st touch only the owner's pixel except in phase 2, where the
 // stores go to pixels outside the list, so no byte store races an atomic or another
 // store to the same byte.
-__device__ bool sweep_owned(uint8_t *st, const FFLists &ls, int L, int Lprev, int *nnext, const float *ph, float *o,
-                            int W, int H)
+__device__ bool sweep_owned(uint8_t *st, const FFLists &ls, int L, int Lprev, int *nnext, volatile int *s_fix,
+                            const float *ph, float *o, int W, int H)
 {
     const int t = threadIdx.x;
     const bool own = t < L;
@@ -520,16 +549,18 @@ __device__ bool sweep_owned(uint8_t *st, const FFLists &ls, int L, int Lprev, in
             if (sn & F_UB) cand = true;
         }
         if (cand) s |= F_CAND | F_NEW;
+        else *s_fix = 1;
         if (s & F_UB) s |= F_NEW;
         st[p] = (uint8_t)s;
     }
     const bool same = __syncthreads_and(all_prev);
+    const bool fix = *s_fix != 0;   // cleared below, behind the next barrier
     for (int e = t; e < Lprev; e += FF_THREADS) {
         const int q = ls.prev[e];
         const unsigned r = st[q];
         if (!(r & F_LIST)) st[q] = (uint8_t)(r & ~F_PREV);
     }
-    for (int guard = 0; guard <= L; guard++) {
+    for (int guard = 0; fix && guard <= L; guard++) {
         bool changed = false;
         if (own && !(s & F_CAND)) {
             bool cand = false;
@@ -573,18 +604,15 @@ __device__ bool sweep_owned(uint8_t *st, const FFLists &ls, int L, int Lprev, in
             }
         }
     }
-    if (__syncthreads_or(wait_dep)) {
+    const bool waits = __syncthreads_or(wait_dep);
+    if (t == 0) *s_fix = 0;
+    if (waits) {
+        const volatile uint8_t *vst = st;
         for (int guard = 0; guard <= L; guard++) {
-            bool done_now = false;
-            if (wait_dep) {
-                const int nb = nbk[kref];
-                if (st[nb] & F_READY) {
-                    o[p] = unwrap_from(o[nb], phv);
-                    done_now = true;
-                }
-            }
-            __syncthreads();
-            if (done_now) {
+            if (wait_dep && (vst[nbk[kref]] & F_READY)) {
+                __threadfence_block();
+                o[p] = unwrap_from(*(volatile const float *)&o[nbk[kref]], phv);
+                __threadfence_block();
                 s |= F_READY;
                 st[p] = (uint8_t)s;
                 wait_dep = false;
@@ -626,12 +654,16 @@ __device__ bool sweep_owned(uint8_t *st, const FFLists &ls, int L, int Lprev, in
 constexpr int FF_SMEM_MAX = 3072, FF_SMEM_CAP = 1024;
 static int g_fill_cap = FF_SMEM_CAP;   // set by ctdm_set_fill_list_capacity
 
+// Bound by the latency of its sweeps (about 500 of them, a few barriers each; DRAM below 1%).
+// 49 maps of 256^2 with residues and cuts: 1003 us with a fixed point and two-barrier rounds
+// in every sweep, 975 with the fixed point only where a pixel needs it and one barrier a
+// round, 916 with the cuts' gather by 8 warps as well.
 // The fill of one map (FloodFill, cTDM/Goldstein.cu:643-1095).  Returns the status (0
 // done, 1 sweep limit, 2 no seed) or -1 when a list outgrew ls.cap.
 // s_cnt[2]: list lengths; the list of sweep j is counted in s_cnt[j & 1] while sweep j
 // counts the next one in s_cnt[(j + 1) & 1].
 __device__ int fill_map(uint8_t *st, const uint8_t *cut, const float *ph, float *o, int W, int H, FFLists ls,
-                        int *s_ok, int *s_cnt)
+                        int *s_ok, int *s_cnt, int *s_fix)
 {
     const int t = threadIdx.x;
     const long n = (long)W * H;
@@ -662,6 +694,7 @@ __device__ int fill_map(uint8_t *st, const uint8_t *cut, const float *ph, float 
             o[seed] = ph[seed];
         }
         *s_ok = ok;
+        *s_fix = 0;
         s_cnt[0] = cnt;
         s_cnt[1] = 0;
     }
@@ -688,7 +721,7 @@ __device__ int fill_map(uint8_t *st, const uint8_t *cut, const float *ph, float 
             if (t == 0) *nnext = 0;
             bool same;
             if (L2 <= FF_THREADS) {
-                same = sweep_owned(st, ls, L2, Lprev, nnext, ph, o, W, H);
+                same = sweep_owned(st, ls, L2, Lprev, nnext, s_fix, ph, o, W, H);
             } else {
                 bool all_prev = true;
                 for (int e = t; e < L2; e += FF_THREADS) {
@@ -765,7 +798,7 @@ __global__ void __launch_bounds__(FF_THREADS) floodfill_kernel(const uint8_t *__
                                                               int smem_cap)
 {
     extern __shared__ __align__(16) uint8_t sstate[];
-    __shared__ int s_ok, s_cnt[2];
+    __shared__ int s_ok, s_cnt[2], s_fix;
     const int a = blockIdx.x;
     const long n = (long)W * H;
     uint8_t *st = SMEM ? sstate : gstate + a * n;
@@ -791,10 +824,10 @@ __global__ void __launch_bounds__(FF_THREADS) floodfill_kernel(const uint8_t *__
         sm.ref = sl + 3 * cap;
         sm.nv = reinterpret_cast<float *>(sl + 4 * cap);
         sm.cap = cap;
-        stat = fill_map(st, cut, ph, o, W, H, sm, &s_ok, s_cnt);
+        stat = fill_map(st, cut, ph, o, W, H, sm, &s_ok, s_cnt, &s_fix);
         __syncthreads();
     }
-    if (stat < 0) stat = fill_map(st, cut, ph, o, W, H, gl, &s_ok, s_cnt);
+    if (stat < 0) stat = fill_map(st, cut, ph, o, W, H, gl, &s_ok, s_cnt, &s_fix);
     if (threadIdx.x == 0) status[a] = stat;
 }
 

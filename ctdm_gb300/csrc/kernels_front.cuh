@@ -68,7 +68,8 @@ cudaError_t stack_to_rytov(const float *ph, const float *am, int A, int R, float
 
 // Goldstein ---------------------------------------------------------------
 cudaError_t goldstein_residues(const float *phi, int A, int W, int H, int8_t *charges, cudaStream_t s);
-cudaError_t goldstein_cuts(const int8_t *charges, int A, int W, int H, uint8_t *cuts, int8_t *work,
+// beside: on a side stream next to the loop (nothing waits for the cuts).
+cudaError_t goldstein_cuts(const int8_t *charges, int A, int W, int H, uint8_t *cuts, int8_t *work, bool beside,
                            cudaStream_t s);
 cudaError_t goldstein_floodfill(const uint8_t *cuts, const float *phi, int A, int W, int H, float *out,
                                 uint8_t *state, int *lists, int *status, cudaStream_t s);
