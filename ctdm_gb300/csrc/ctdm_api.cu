@@ -732,14 +732,15 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
     }
     la.xprev = nullptr;
     la.beta = 0.f;
-    if (accelerated && iters > 0) {
+    if (accelerated && iters > 1) {   // one iteration has no previous iterate: the plain loop's
         CK(ensure(c, B_XPREV, sizeof(float2) * (size_t)R * R * R), "alloc accelerated iterate");
         la.xprev = B<float2>(c, B_XPREV);
     }
     double t_k = 1.0;
-    auto next_beta = [&]() {   // beta of this iteration (0 for the first: x_{-1} is not used)
+    auto next_beta = [&](int it) {   // beta of this iteration (0 for the first: x_{-1} is not used)
         const double t_n = 0.5 * (1.0 + std::sqrt(1.0 + 4.0 * t_k * t_k));
         la.beta = (float)((t_k - 1.0) / t_n);
+        if (la.xprev) la.mom = it == 0 ? MOM_FIRST : it + 1 == iters ? MOM_LAST : MOM_STEP;
         t_k = t_n;
     };
     StageTimer &tm = c->timer;
@@ -751,7 +752,7 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
         // plane + z passes, 8- or 4-CTA clusters per plane (schemes 1, 2; the plane pass
         // records under the x-pass stage)
         for (int it = 0; it < iters; it++) {
-            next_beta();
+            next_beta(it);
             CK(launch_plane(la, false, s), "plane pass");
             tm.mark(S_XPASS, s);
             CK(launch_zpass(la, check_mode, s), "z pass");
@@ -767,7 +768,7 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
     la.xactive = xactive;
     tm.mark(S_YINV, s);
     for (int it = 0; it < iters; it++) {
-        next_beta();
+        next_beta(it);
         CK(launch_xpass(la, false, s), "x pass");
         tm.mark(S_XPASS, s);
         CK(launch_ypass(la, false, s), "y forward pass");

@@ -78,6 +78,10 @@ struct EwaldArgs {
     const int *fi_frame;
 };
 
+// What an iteration does with the previous iterate: the first has none to read, after the
+// last nobody reads the one it would store.
+enum Momentum { MOM_NONE, MOM_FIRST, MOM_STEP, MOM_LAST };
+
 struct LoopArgs {
     float2 *G;
     const float2 *F2;
@@ -110,6 +114,7 @@ struct LoopArgs {
     // to the forward transform; xprev == nullptr: the plain loop
     float2 *xprev;
     float beta;
+    int mom;   // Momentum of this iteration
 };
 
 // Whether the loop of side R leaves out what no measured voxel touches (loop_passes.cuh).

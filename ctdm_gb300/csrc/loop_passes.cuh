@@ -92,7 +92,8 @@ __device__ __forceinline__ void prefetch_lines(const float2 *G, long ln)
 // its first-stage points straight from HBM (unit stride across the warp), the
 // inverse transform ends in registers, the point operators run on the registers,
 // and the forward transform in the reversed radix order stores straight back.
-template <class P, bool FINAL, bool MOM = false>
+// MOM: the iteration's Momentum (the last iteration runs as any other).
+template <class P, bool FINAL, int MOM = MOM_NONE>
 __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4)) xpass_kernel(LoopArgs a,
                                                                                       const float2 *__restrict__ tw)
 {
@@ -103,7 +104,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4)) xpass_k
     const int t = threadIdx.x % P::T, b = threadIdx.x / P::T;
     const long l = (long)blockIdx.x * P::B + b;   // row y + L z (the grid covers the L^2 rows exactly)
     const float2 *src = a.G + l * L;
-    if constexpr (MOM && !FINAL) {
+    if constexpr (MOM == MOM_STEP && !FINAL) {
         // the previous iterate of this row comes from HBM during the inverse transform
 #pragma unroll
         for (int i = 0; i < P::E; i++) prefetch_l2(a.xprev + l * L + fftl::slot_pos<L, P::T, P::RV0>(i, t));
@@ -129,9 +130,13 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4)) xpass_k
 #pragma unroll
             for (int i = 0; i < P::E; i++) {
                 const int o = fftl::slot_pos<L, P::T, P::RV0>(i, t);
-                const float2 prev = xp[o];
-                xp[o] = v[i];
-                v[i] = momentum_step(v[i], prev, a.beta);
+                if constexpr (MOM == MOM_FIRST) {
+                    xp[o] = v[i];   // beta 0: what is sent on is the iterate itself
+                } else {
+                    const float2 prev = xp[o];
+                    xp[o] = v[i];
+                    v[i] = momentum_step(v[i], prev, a.beta);
+                }
             }
         }
         P::template seqr_row<false>(buf, v, tw);
@@ -377,7 +382,9 @@ static cudaError_t run_loop_pass(int kind, const LoopArgs &a, int flag, cudaStre
     if (kind == LOOP_X || kind == LOOP_X_FINAL) {
         const size_t smem = fftl::plan_smem_row<P>();
         auto k = kind == LOOP_X_FINAL ? xpass_kernel<P, true>
-                                      : (a.xprev ? xpass_kernel<P, false, true> : xpass_kernel<P, false>);
+                                      : (a.mom == MOM_NONE ? xpass_kernel<P, false>
+                                         : (a.mom == MOM_FIRST ? xpass_kernel<P, false, MOM_FIRST>
+                                                               : xpass_kernel<P, false, MOM_STEP>));
         e = prep_plan_kernel(k, L, smem);
         if (e != cudaSuccess) return e;
         return launch_pass<L>(k, grid, P::THREADS, smem, s, a, twiddles(L));

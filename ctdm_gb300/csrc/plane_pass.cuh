@@ -23,7 +23,6 @@
 #include "tma.cuh"
 
 namespace ctdm {
-
 // PP: the line plan (lines per CTA, threads per line, radices) of the rows and columns.
 template <int L, int C, class PP = fftl::Plan<L>>
 struct PlaneCfg {
@@ -37,8 +36,9 @@ struct PlaneCfg {
 
 // MINB: resident CTAs per SM the register allocation aims for (3: no spills at
 // R = 256; 4: more latency hiding for some spill traffic).  C: CTAs per plane.
-// MOM: the accelerated loop (momentum on the projected iterate, LoopArgs::xprev).
-template <int L, int C, int MINB, bool FINAL, bool MOM = false, class PP = fftl::Plan<L>>
+// MOM: the accelerated loop (momentum on the projected iterate, LoopArgs::xprev), by the
+// iteration's Momentum.
+template <int L, int C, int MINB, bool FINAL, int MOM = MOM_NONE, class PP = fftl::Plan<L>>
 __global__ void __launch_bounds__(PP::THREADS, MINB) plane_kernel(LoopArgs a, const float2 *__restrict__ tw)
 {
     namespace cg = cooperative_groups;
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(PP::THREADS, MINB) plane_kernel(LoopArgs a, co
         for (int sb = 0; sb < Cfg::SB; sb++) {
             const int x = rank * RL + sb * P::B + b;
             float2 *col = plane + x;
-            if constexpr (MOM && !FINAL) {
+            if constexpr ((MOM == MOM_STEP || MOM == MOM_LAST) && !FINAL) {
                 // the previous iterate of these columns comes from HBM during the transform
                 const float2 *xp = a.xprev + (long)z * L * L + x;
 #pragma unroll
@@ -95,17 +95,33 @@ __global__ void __launch_bounds__(PP::THREADS, MINB) plane_kernel(LoopArgs a, co
                     dst[(long)L * ((y + L / 2) % L)] = est_n_scaled(v[i], a.s1, a.n_med);
                 }
             } else {
-#pragma unroll
-                for (int i = 0; i < P::E; i++) v[i] = modify_f_scaled(est_n_scaled(v[i], a.s1, a.n_med), a.s2, a.k2);
-                if constexpr (MOM) {
+                if constexpr (MOM == MOM_FIRST) {
+                    // beta 0: what is sent on is the iterate itself
                     float2 *xp = a.xprev + (long)z * L * L + x;
 #pragma unroll
                     for (int i = 0; i < P::E; i++) {
-                        const long o = (long)L * fftl::slot_pos<L, P::T, P::RV0>(i, t);
-                        const float2 prev = xp[o];
-                        xp[o] = v[i];
-                        v[i] = momentum_step(v[i], prev, a.beta);
+                        v[i] = modify_f_scaled(est_n_scaled(v[i], a.s1, a.n_med), a.s2, a.k2);
+                        __stcs(&xp[(long)L * fftl::slot_pos<L, P::T, P::RV0>(i, t)], v[i]);
                     }
+                } else if constexpr (MOM) {
+                    // the previous iterate is loaded whole before any of the new one is stored:
+                    // with load and store in turn (they may alias, as far as the compiler knows)
+                    // ten iterations took 2.11 / 8.23 / 20.8 ms at 256 / 384 / 512, so 1.94 /
+                    // 8.11 / 20.3; without the first load and the last store 1.94 / 8.09 / 20.0.
+                    float2 *xp = a.xprev + (long)z * L * L + x;
+                    float2 prev[P::E];
+#pragma unroll
+                    for (int i = 0; i < P::E; i++) prev[i] = __ldcs(&xp[(long)L * fftl::slot_pos<L, P::T, P::RV0>(i, t)]);
+#pragma unroll
+                    for (int i = 0; i < P::E; i++) v[i] = modify_f_scaled(est_n_scaled(v[i], a.s1, a.n_med), a.s2, a.k2);
+#pragma unroll
+                    for (int i = 0; i < P::E; i++) {
+                        if constexpr (MOM != MOM_LAST) __stcs(&xp[(long)L * fftl::slot_pos<L, P::T, P::RV0>(i, t)], v[i]);
+                        v[i] = momentum_step(v[i], prev[i], a.beta);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < P::E; i++) v[i] = modify_f_scaled(est_n_scaled(v[i], a.s1, a.n_med), a.s2, a.k2);
                 }
                 P::template seqr<false, false, false>(scr, v, tw);
 #pragma unroll
@@ -137,8 +153,11 @@ template <int L, int C, int MINB, class PP = fftl::Plan<L>>
 static cudaError_t run_plane_pass(const LoopArgs &a, bool final_pass, cudaStream_t s)
 {
     using Cfg = PlaneCfg<L, C, PP>;
-    auto k = final_pass ? plane_kernel<L, C, MINB, true, false, PP>
-                        : (a.xprev ? plane_kernel<L, C, MINB, false, true, PP> : plane_kernel<L, C, MINB, false, false, PP>);
+    auto k = plane_kernel<L, C, MINB, false, MOM_NONE, PP>;
+    if (final_pass) k = plane_kernel<L, C, MINB, true, MOM_NONE, PP>;
+    else if (a.mom == MOM_FIRST) k = plane_kernel<L, C, MINB, false, MOM_FIRST, PP>;
+    else if (a.mom == MOM_STEP) k = plane_kernel<L, C, MINB, false, MOM_STEP, PP>;
+    else if (a.mom == MOM_LAST) k = plane_kernel<L, C, MINB, false, MOM_LAST, PP>;
     if (!twiddles(L)) return cudaErrorInitializationError;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -173,7 +192,7 @@ template <int L, int C, int MINB, class PP = fftl::Plan<L>>
 static int plane_pass_clusters()
 {
     using Cfg = PlaneCfg<L, C, PP>;
-    auto k = plane_kernel<L, C, MINB, false, false, PP>;
+    auto k = plane_kernel<L, C, MINB, false, MOM_NONE, PP>;
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::SMEM) != cudaSuccess) return 0;
     if (C > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return 0;
     cudaLaunchConfig_t cfg = {};
