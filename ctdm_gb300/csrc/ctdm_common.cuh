@@ -31,7 +31,7 @@ __device__ __forceinline__ float2 cmul_mi(float2 a)
 // loop-invariant, they are not kept in registers across it (15 complex values per radix-16
 // stage cost more than reloading them from L1).
 template <class T>
-__device__ __forceinline__ const T *fresh(const T *p)
+__device__ __forceinline__ T *fresh(T *p)
 {
     asm volatile("" : "+l"(p));
     return p;

@@ -130,6 +130,7 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
     namespace cg = cooperative_groups;
     chain_begin();
     phi = fresh(phi);
+    T = fresh(T);
     using Y = fftl::Lay<M, P::LP, true>;
     constexpr int RPC = M / C, RL = 2 * P::B, E = P::E;
     static_assert(RPC % RL == 0 && P::T <= 32, "whole steps per CTA, a line within a warp");
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
                     const int e = tid + k * P::THREADS;
                     const int y = yh - 1 + e / M;
                     if (e < (P::B + 2) * M)
-                        S[e] = (y >= 0 && y < M) ? __ldg(phi + map + (long)(yh - 1) * M + e) : 0.f;
+                        S[e] = (y >= 0 && y < M) ? __ldca(phi + map + (long)(yh - 1) * M + e) : 0.f;
                 }
                 __syncthreads();
 #pragma unroll 2

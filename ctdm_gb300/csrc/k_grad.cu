@@ -241,6 +241,7 @@ __global__ void __launch_bounds__(P::THREADS, P::E <= 16 ? 1024 / P::THREADS : 5
     tape_z_kernel(TapeZ a, const float2 *__restrict__ tw)
 {
     chain_begin();
+    a.G = fresh(a.G);
     constexpr bool RES = MODE == Z_RESIDUAL || MODE == Z_RESIDUAL_SUM;
     constexpr int L = P::L;
     static_assert(P::B <= 32 && P::B <= L, "one mask word per z row of a tile");
@@ -420,6 +421,8 @@ template <bool UPDATE>
 __global__ void __launch_bounds__(kTvThreads, 3) tv_kernel(TvArgs a)
 {
     chain_begin();
+    a.W = fresh(a.W);
+    const float2 *gin = fresh(a.g), *vin = fresh(a.V);
     __shared__ float2 pl[2][kTvH][kTvW];           // planes z and z + 1, one-voxel halo
     __shared__ float2 qx[kTvY][kTvX + 1], qy[kTvY + 1][kTvX];   // q of the tile and its x / y halo
     const int R = a.R, nbx = R / kTvX, nby = R / kTvY;
@@ -440,7 +443,7 @@ __global__ void __launch_bounds__(kTvThreads, 3) tv_kernel(TvArgs a)
         const float2 *p = a.W + (long)rr * min(max(z, 0), R - 1);
 #pragma unroll
         for (int j = 0; j < kTvLoads; j++)
-            if (off[j] >= 0) r[j] = __ldg(p + off[j]);
+            if (off[j] >= 0) r[j] = __ldca(p + off[j]);
     };
     auto put = [&](float2 *plane, const float2 *r) {
 #pragma unroll
@@ -466,8 +469,8 @@ __global__ void __launch_bounds__(kTvThreads, 3) tv_kernel(TvArgs a)
         if (own) {   // in flight while q is computed
 #pragma unroll
             for (int h = 0; h < 2; h++) {
-                gv[h] = __ldcs(&a.g[i0 + 8 * h * R]);
-                if constexpr (UPDATE) vv[h] = __ldcs(&a.V[i0 + 8 * h * R]);
+                gv[h] = __ldcs(&gin[i0 + 8 * h * R]);
+                if constexpr (UPDATE) vv[h] = __ldcs(&vin[i0 + 8 * h * R]);
             }
         }
 #pragma unroll

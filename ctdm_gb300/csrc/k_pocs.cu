@@ -114,7 +114,7 @@ constexpr int kPer = 4;
 // takes 290 us (a third of it the projection's roots and divisions).
 struct LoadReal {
     const float *p;
-    __device__ __forceinline__ float2 operator()(long i) const { return make_float2(__ldg(p + i), 0.f); }
+    __device__ __forceinline__ float2 operator()(long i) const { return make_float2(__ldca(p + i), 0.f); }
 };
 
 constexpr int kTileVals = 512;   // packed values staged per tile

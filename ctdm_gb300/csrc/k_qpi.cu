@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) carrier_argmax_kernel(const float2 *__res
 // Forward row transforms of real rows (the image is read as it is).
 struct LoadRealRow {
     const float *p;
-    __device__ __forceinline__ float2 operator()(long i) const { return make_float2(__ldg(p + i), 0.f); }
+    __device__ __forceinline__ float2 operator()(long i) const { return make_float2(__ldca(p + i), 0.f); }
 };
 template <int L>
 static cudaError_t rows_real_launch(const float *src, float2 *dst, long nlines, cudaStream_t s)
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(QRows<N>::THREADS, 1024 / QRows<N>::THREADS)
     // Only the columns of the radius box survive the column pass's mask: window
     // columns m in [mlo, mhi] (|m - M/2| <= radius), spectrum columns k in
     // [kb, kb + W) mod N.  Park those points and their mirrors.
-    const int c = __ldg(&carrier[1]), rad = __ldg(&carrier[2]);
+    const int c = __ldca(&carrier[1]), rad = __ldca(&carrier[2]);
     const int mlo = max(0, M / 2 - rad), mhi = min(M - 1, M / 2 + rad), W = mhi - mlo + 1;
     const int kb = (c - N / 2 - M / 2 + mlo + 2 * N) & (N - 1);
 #pragma unroll
@@ -257,12 +257,13 @@ __global__ void __launch_bounds__(Plan<M>::THREADS) qpi_rows_inv_kernel(float2 *
                                                                        const float2 *__restrict__ tw)
 {
     chain_begin();
+    S = fresh(S);
     carrier = fresh(carrier);
     using P = Plan<M>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
     const long line0 = (long)blockIdx.x * P::B;
-    const int rad = __ldg(&carrier[2]);
+    const int rad = __ldca(&carrier[2]);
     bool any_in = false;   // the same for every thread of the CTA
     for (int bb = 0; bb < P::B; bb++) {
         const long lb = line0 + bb;
@@ -328,7 +329,7 @@ __global__ void __launch_bounds__(Plan<M>::THREADS) qpi_final_kernel(const float
     const long a = ok ? l / M : 0;
     const long mm = (long)M * M;
     const float2 *src = S + a * mm + x;
-    const int rad = __ldg(&carrier[2]);
+    const int rad = __ldca(&carrier[2]);
     float2 v[P::E];
 #pragma unroll
     for (int i = 0; i < P::E; i++) {
@@ -446,10 +447,10 @@ __device__ __forceinline__ float qpib_tap(const float *__restrict__ h, int N, fl
 {
     const int ix = (int)(xr * (float)i), iy = (int)(yr * (float)j);
     const float a = xr * (float)i - (float)ix, b = yr * (float)j - (float)iy;
-    const float d00 = (ix < N && iy < N) ? __ldg(&h[(long)iy * N + ix]) : 0.f;
-    const float d10 = (ix + 1 < N && iy < N) ? __ldg(&h[(long)iy * N + ix + 1]) : 0.f;
-    const float d01 = (ix < N && iy + 1 < N) ? __ldg(&h[(long)(iy + 1) * N + ix]) : 0.f;
-    const float d11 = (ix + 1 < N && iy + 1 < N) ? __ldg(&h[(long)(iy + 1) * N + ix + 1]) : 0.f;
+    const float d00 = (ix < N && iy < N) ? __ldca(&h[(long)iy * N + ix]) : 0.f;
+    const float d10 = (ix + 1 < N && iy < N) ? __ldca(&h[(long)iy * N + ix + 1]) : 0.f;
+    const float d01 = (ix < N && iy + 1 < N) ? __ldca(&h[(long)(iy + 1) * N + ix]) : 0.f;
+    const float d11 = (ix + 1 < N && iy + 1 < N) ? __ldca(&h[(long)(iy + 1) * N + ix + 1]) : 0.f;
     const float t1 = a * d10 + (-d00 * a + d00);
     const float t2 = a * d11 + (-d01 * a + d01);
     return b * t2 + (-t1 * b + t1);
@@ -541,7 +542,7 @@ __global__ void __launch_bounds__(1024) qpib_center_kernel(const float *__restri
     for (int j0 = 0; j0 < H; j0 += step) {
         const int rows = min(step, H - j0);
         __syncthreads();
-        for (int e = threadIdx.x; e < rows * nc; e += 1024) srow[e] = __ldg(&mag[(long)(j0 + e / nc) * N + lo + e % nc]);
+        for (int e = threadIdx.x; e < rows * nc; e += 1024) srow[e] = __ldca(&mag[(long)(j0 + e / nc) * N + lo + e % nc]);
         __syncthreads();
         if ((int)threadIdx.x < nc) {
 #pragma unroll 8

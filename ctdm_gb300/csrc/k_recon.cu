@@ -88,6 +88,7 @@ __global__ void __launch_bounds__(ColPlan<L>::THREADS) cols_kernel(const float2 
                                                                    const int *__restrict__ xactive)
 {
     chain_begin();
+    src = fresh(src);
     xactive = fresh(xactive);
     using P = ColPlan<L>;
     extern __shared__ float4 smem4[];
@@ -95,7 +96,7 @@ __global__ void __launch_bounds__(ColPlan<L>::THREADS) cols_kernel(const float2 
     const long line0 = (long)blockIdx.x * P::B;
     if (xactive) {
         int any = 0;
-        for (int x = 0; x < (P::B < nx ? P::B : nx); x += 8) any |= __ldg(&xactive[(line0 % nx + x) / 8]);
+        for (int x = 0; x < (P::B < nx ? P::B : nx); x += 8) any |= __ldca(&xactive[(line0 % nx + x) / 8]);
         if (!any) return;
     }
     bool ok;
@@ -237,9 +238,9 @@ __device__ __forceinline__ float2 fi_sample(int ii, int jj, int nzs, double df, 
         s = lo;
         w = (tp - th[lo]) / (th[hi] - th[lo]);
     }
-    float2 u = __ldg(&ucol[fr[s] * rr]);
+    float2 u = __ldca(&ucol[fr[s] * rr]);
     if (w > 0.0) {
-        const float2 u2 = __ldg(&ucol[fr[s + 1] * rr]);
+        const float2 u2 = __ldca(&ucol[fr[s + 1] * rr]);
         const float wf = (float)w, vf = (float)(1.0 - w);
         u = make_float2(vf * u.x + wf * u2.x, vf * u.y + wf * u2.y);
     }
@@ -300,6 +301,7 @@ __global__ void __launch_bounds__(EwaldCfg<P, ZINV>::THREADS)
     ewald_kernel(EwaldArgs a, EwaldRange rg, unsigned body, const float2 *__restrict__ tw)
 {
     chain_begin();
+    a.U = fresh(a.U);
     constexpr int R = P::L, B = EwaldCfg<P, ZINV>::B, THREADS = EwaldCfg<P, ZINV>::THREADS;
     extern __shared__ float4 smem4[];
     float2 *acc = reinterpret_cast<float2 *>(smem4);                    // [plane][column]
@@ -339,7 +341,7 @@ __global__ void __launch_bounds__(EwaldCfg<P, ZINV>::THREADS)
             if (ang >= a.A || !geo[ang].valid) return -1;
             const int nzs = ewald_nz_signed(ii, jj, geo[ang], a.df, a.fm02, a.fm02s, fz);
             if (nzs == kNoSample) return -1;
-            u = __ldg(&ucol[ang * rr]);
+            u = __ldca(&ucol[ang * rr]);
             if constexpr (FI)
                 u = fi_sample(ii, jj, nzs, a.df, a.fm0, asin(geo[ang].fy0 / a.fm0), th, fr, a.A, ucol, rr, u, fz);
             const int slot = imod(nzs - rg.lo, R);

@@ -289,8 +289,8 @@ __global__ void __launch_bounds__(256) prep_resize_kernel(const float *__restric
         const float a = xr * (float)i - (float)ix;
         const bool in0 = ix < M && y < M, in1 = ix + 1 < M && y < M;
         const long o = (long)y * M + ix;
-        const float p0 = in0 ? __ldg(&P[o]) : 0.f, p1 = in1 ? __ldg(&P[o + 1]) : 0.f;
-        const float a0 = in0 ? __ldg(&Am[o]) : 0.f, a1 = in1 ? __ldg(&Am[o + 1]) : 0.f;
+        const float p0 = in0 ? __ldca(&P[o]) : 0.f, p1 = in1 ? __ldca(&P[o + 1]) : 0.f;
+        const float a0 = in0 ? __ldca(&Am[o]) : 0.f, a1 = in1 ? __ldca(&Am[o + 1]) : 0.f;
         odd |= !(fmaxf(fmaxf(fabsf(p0), fabsf(p1)), fmaxf(fabsf(a0), fabsf(a1))) < 1e30f) || isnan(p0 + p1) ||
                isnan(a0 + a1);
         hp[r][c] = a * p1 + (-p0 * a + p0);

@@ -24,10 +24,19 @@ const float *dct_eigen(int M);
 // A kernel that starts with chain_begin() may be launched with launch_chained: its CTAs are
 // then scheduled while the last ones of the kernel before it in the stream still run, and
 // wait in chain_begin until that kernel has completed and its writes are visible, so that
-// the launch latency is hidden.  Nothing but the tables is read or written before
-// chain_begin, and const __restrict__ inputs go through fresh() after it, so that the
-// compiler cannot take their loads for invariant and move them ahead.  (Every
-// kernel of a chain waits for the one before it, so the wait covers all earlier ones.)
+// the launch latency is hidden.  (Every kernel of a chain waits for the one before it, so the
+// wait covers all earlier ones.)  A chained kernel lives while its input is still being
+// written, so
+//   - nothing but the tables is read or written before chain_begin;
+//   - pointers to what earlier launches write, parameters and struct members alike, go
+//     through fresh() after it where they are const __restrict__ or read by a load intrinsic:
+//     the compiler may move such loads ahead of the wait otherwise;
+//   - those loads are __ldca, __ldcs or __ldcg, never __ldg: the read-only path asks for
+//     memory that does not change during the whole kernel.  __ldg is for tables and for what
+//     was complete before the chain's first launch (a tape's sample lists).  (Not plain loads
+//     in a loop: behind fresh() the compiler no longer knows that they are global, and keeps
+//     them in order with stores to shared memory; 121 maps of 256^2 unwrapped in 133 us so
+//     instead of 110.)
 __device__ __forceinline__ void chain_begin()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

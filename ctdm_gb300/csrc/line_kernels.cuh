@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(P::THREADS, row_min_ctas<P>())
     rows_fn_kernel(LD ld, ST st, const float2 *__restrict__ tw, long nlines)
 {
     chain_begin();
+    ld.p = fresh(ld.p);
     constexpr int L = P::L;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);

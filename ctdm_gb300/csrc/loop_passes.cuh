@@ -47,6 +47,15 @@ static cudaError_t prep_plan_kernel(K kernel, int L, size_t smem)
 // next one another 1.3; five loop bodies with the chained front end went from 248 to 202 us
 // (16 x 256^2 frames -> 64^3).  At 256^3 a pass hides nothing that shows.
 constexpr bool chain_passes(int L) { return L <= 128; }
+template <int L>
+__device__ __forceinline__ void chain_pass(LoopArgs &a)
+{
+    if constexpr (chain_passes(L)) {
+        chain_begin();
+        a.G = fresh(a.G);
+        a.F2 = fresh(a.F2);
+    }
+}
 
 // Lines one wave ahead for a z-pass kernel: its resident CTAs on the device x lines per
 // CTA (0 when the occupancy query fails), once per kernel and device.  A z-pass CTA
@@ -98,7 +107,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4)) xpass_k
                                                                                       const float2 *__restrict__ tw)
 {
     constexpr int L = P::L;
-    if constexpr (chain_passes(L)) chain_begin();
+    chain_pass<L>(a);
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
     const int t = threadIdx.x % P::T, b = threadIdx.x / P::T;
@@ -156,7 +165,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(5)) ypass_k
                                                                                       const float2 *__restrict__ tw)
 {
     constexpr int L = P::L;
-    if constexpr (chain_passes(L)) chain_begin();
+    chain_pass<L>(a);
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
     // planes in descending z: the x pass runs them ascending, so each pass starts on
@@ -169,7 +178,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(5)) ypass_k
         int any = 0;   // the same for every thread: a CTA's B columns share one z
         const int x0 = (int)(line0 % L);
 #pragma unroll
-        for (int x = 0; x < (P::B < L ? P::B : L); x += 8) any |= __ldg(&a.xactive[(x0 + x) / 8]);
+        for (int x = 0; x < (P::B < L ? P::B : L); x += 8) any |= a.xactive[(x0 + x) / 8];
         if (!any) return;
     }
     float2 v[P::E];
@@ -211,7 +220,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(3))
     constexpr int L = P::L;
     constexpr bool TMA = zpass_tma<P>();
     const bool staged = TMA && a.staged;   // uniform over the grid
-    if constexpr (chain_passes(L)) chain_begin();
+    chain_pass<L>(a);
     extern __shared__ float4 smem4[];
     // [F2 tile, z-major: B*L float2][mask tile B*L bytes][FFT buffer][mbarrier], 128-byte aligned
     char *base0 = reinterpret_cast<char *>(smem4);
@@ -305,7 +314,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4))
     zpass_packed_kernel(LoopArgs a, const float2 *__restrict__ tw, int ahead)
 {
     constexpr int L = P::L;
-    if constexpr (chain_passes(L)) chain_begin();
+    chain_pass<L>(a);
     extern __shared__ float4 smem4[];
     char *base0 = reinterpret_cast<char *>(smem4);
     char *al = base0 + ((128 - (tma::smem_addr(base0) & 127)) & 127);
@@ -316,9 +325,9 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4))
     uint64_t *bar = reinterpret_cast<uint64_t *>(buf + P::B * P::LP);
     const long nl = (long)L * L;
     constexpr bool SKIP = skip_empty_tiles(L);
-    const int nact = SKIP ? __ldg(a.zcount) : (int)gridDim.x;
+    const int nact = SKIP ? *a.zcount : (int)gridDim.x;
     if ((int)blockIdx.x >= nact) return;
-    const long tile = SKIP ? __ldg(&a.ztiles[blockIdx.x]) : (long)blockIdx.x;
+    const long tile = SKIP ? a.ztiles[blockIdx.x] : (long)blockIdx.x;
     const long line0 = tile * P::B;   // line = x + L y
     if (threadIdx.x == 0) {
         tma::mbar_init(bar, 1);
@@ -336,7 +345,7 @@ __global__ void __launch_bounds__(P::THREADS, fftl::plan_min_ctas<P>(4))
     const int b = threadIdx.x % P::B, t = threadIdx.x / P::B;
     const long base = line0 + b;
     if (ahead > 0 && (int)blockIdx.x + ahead < nact)
-        prefetch_lines<P>(a.G, (SKIP ? (long)__ldg(&a.ztiles[blockIdx.x + ahead]) : (long)blockIdx.x + ahead) * P::B);
+        prefetch_lines<P>(a.G, (SKIP ? (long)a.ztiles[blockIdx.x + ahead] : (long)blockIdx.x + ahead) * P::B);
     float2 v[P::E];
 #pragma unroll
     for (int i = 0; i < P::E; i++) v[i] = __ldcs(&a.G[base + (long)fftl::slot_pos<L, P::T, P::F0>(i, t) * nl]);
