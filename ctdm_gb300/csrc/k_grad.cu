@@ -802,8 +802,9 @@ extern "C" ctdm_status ctdm_loss_grad(ctdm_tape *t, const ctdm_cfloat *d_V, doub
     const float2 *V = reinterpret_cast<const float2 *>(d_V);
     cudaError_t e = residual_xspace(t, V, true, 0);
     double data = 0, tv = 0;
-    if (e == cudaSuccess) data = 0.5 * sum_partials(t->red, t->tiles);
     if (e == cudaSuccess) e = rows_adjoint(t)(t->work, grad, unitary_scale(t), 0);
+    // the sums come last: reading one back is what the call waits for
+    if (e == cudaSuccess) data = 0.5 * sum_partials(t->red, t->tiles);
     if (e == cudaSuccess && lambda != 0.0) {
         TvArgs a = {};
         a.W = V;
