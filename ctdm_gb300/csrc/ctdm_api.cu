@@ -712,7 +712,8 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
     CK(ensure_tuned(R, check_mode, s), "autotune loop passes");
     // B_TACT: the caller made it and cleared its header
     // the z pass reads the measured samples packed per tile when its plan allows
-    const int TB = loop_ztile(R);
+    const LoopPlan lp = loop_plan(R);
+    const int TB = lp.ztile;
     la.packed = 0;
     if (TB > 0) {
         const long r3 = (long)R * R * R, tiles = (long)R * R / TB;
@@ -746,39 +747,39 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
     StageTimer &tm = c->timer;
     // where empty tiles are skipped G holds z lines normalised by 1 / R (loop_g_scale, the z
     // passes) and the y inverse line pass normalises too; the rest is left to s1
-    const bool planes = loop_scheme(R) >= 1;
+    const bool planes = lp.scheme >= 1;
     la.s1 = (float)(-1.0 / ((!skip_empty_tiles(R) ? (double)R * R * R : planes ? (double)R * R : (double)R) * k2));
     if (planes) {
         // plane + z passes, 8- or 4-CTA clusters per plane (schemes 1, 2; the plane pass
         // records under the x-pass stage)
         for (int it = 0; it < iters; it++) {
             next_beta(it);
-            CK(launch_plane(la, false, s), "plane pass");
+            CK(launch_plane(lp, la, false, s), "plane pass");
             tm.mark(S_XPASS, s);
-            CK(launch_zpass(la, check_mode, s), "z pass");
+            CK(launch_zpass(lp, la, check_mode, s), "z pass");
             tm.mark(S_ZPASS, s);
         }
-        CK(launch_plane(la, true, s), "final plane pass");
+        CK(launch_plane(lp, la, true, s), "final plane pass");
         tm.mark(S_XFINAL, s);
         return CTDM_OK;
     }
     const int *xactive = la.xactive;
     la.xactive = nullptr;   // F2 may hold values that the loop does not keep: every column
-    CK(launch_ypass(la, true, s), "y inverse pass");
+    CK(launch_ypass(lp, la, true, s), "y inverse pass");
     la.xactive = xactive;
     tm.mark(S_YINV, s);
     for (int it = 0; it < iters; it++) {
         next_beta(it);
-        CK(launch_xpass(la, false, s), "x pass");
+        CK(launch_xpass(lp, la, false, s), "x pass");
         tm.mark(S_XPASS, s);
-        CK(launch_ypass(la, false, s), "y forward pass");
+        CK(launch_ypass(lp, la, false, s), "y forward pass");
         tm.mark(S_YFWD, s);
-        CK(launch_zpass(la, check_mode, s), "z pass");
+        CK(launch_zpass(lp, la, check_mode, s), "z pass");
         tm.mark(S_ZPASS, s);
-        CK(launch_ypass(la, true, s), "y inverse pass");
+        CK(launch_ypass(lp, la, true, s), "y inverse pass");
         tm.mark(S_YINV, s);
     }
-    CK(launch_xpass(la, true, s), "final x pass");
+    CK(launch_xpass(lp, la, true, s), "final x pass");
     tm.mark(S_XFINAL, s);
     return CTDM_OK;
 }

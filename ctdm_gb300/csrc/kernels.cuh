@@ -150,9 +150,19 @@ inline void active_view(LoopArgs &a, const int *active, int R)
 }
 
 cudaError_t launch_ewald(const EwaldArgs &a, cudaStream_t s);
-cudaError_t launch_xpass(const LoopArgs &a, bool final_pass, cudaStream_t s);
-cudaError_t launch_ypass(const LoopArgs &a, bool inverse, cudaStream_t s);
-cudaError_t launch_zpass(const LoopArgs &a, int check_mode, cudaStream_t s);
+// Plan variants of a loop call's passes.  A call reads them once and launches all its passes
+// with them: any thread may tune or pin a side at any time, while the packed tiles have the
+// z variant's width, and the forward and inverse y passes leave out columns by the y
+// variant's lines per CTA.
+struct LoopPlan {
+    int v[3];     // x, y, z pass
+    int scheme;   // loop_scheme
+    int ztile;    // lines per z-pass CTA when that variant reads packed measured samples, else 0
+};
+LoopPlan loop_plan(int R);
+cudaError_t launch_xpass(const LoopPlan &p, const LoopArgs &a, bool final_pass, cudaStream_t s);
+cudaError_t launch_ypass(const LoopPlan &p, const LoopArgs &a, bool inverse, cudaStream_t s);
+cudaError_t launch_zpass(const LoopPlan &p, const LoopArgs &a, int check_mode, cudaStream_t s);
 
 // Positivity-loop passes by plan variant (one translation unit per volume side).
 enum LoopKind { LOOP_X = 0, LOOP_X_FINAL = 1, LOOP_Y_FWD = 2, LOOP_Y_INV = 3, LOOP_Z = 4 };
@@ -170,9 +180,6 @@ int loop_ztile_256(int variant);
 int loop_ztile_384(int variant);
 int loop_ztile_512(int variant);
 int loop_ztile_768(int variant);
-// Tile width (lines per CTA) of the z pass in use for side R when it reads packed
-// measured samples, else 0.
-int loop_ztile(int R);
 // Number of plan variants of the loop passes for volume side R (0: unsupported).
 int loop_plan_count(int R);
 cudaError_t loop_pass_variant(int kind, int variant, const LoopArgs &a, int flag, cudaStream_t s);
@@ -193,7 +200,7 @@ int plane_clusters_512();
 // Loop scheme of side R on this device: 0 = x / y / z / y passes, 1 and 2 = plane + z
 // passes (two cluster sizes per plane: 8 and 4 CTAs at R = 256, 8 and 6 at 384, 16 and 8 at 512).
 int loop_scheme(int R);
-cudaError_t launch_plane(const LoopArgs &a, bool final_pass, cudaStream_t s);
+cudaError_t launch_plane(const LoopPlan &p, const LoopArgs &a, bool final_pass, cudaStream_t s);
 
 // ---- ASD-POCS with total-variation steepest descent (k_pocs.cu)
 // Controller of one run in device memory: kernels read the step sizes from it and the

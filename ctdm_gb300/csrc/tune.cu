@@ -65,8 +65,6 @@ cudaError_t loop_pass_variant(int kind, int variant, const LoopArgs &a, int flag
     }
 }
 
-static PlanChoice choice_of(int R);
-
 // Lines per packed z-pass tile of variant v at side R (0: that plan reads F2 densely).
 static int ztile_of(int R, int v)
 {
@@ -82,19 +80,6 @@ static int ztile_of(int R, int v)
     case 768: return loop_ztile_768(v);
     default: return 0;
     }
-}
-
-int loop_ztile(int R)
-{
-    int v = 0;
-    {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_choice.find({dev, R});
-        if (it != g_choice.end()) v = it->second.v[2];
-    }
-    return ztile_of(R, v);
 }
 
 static PlanChoice choice_of(int R)
@@ -124,11 +109,18 @@ static bool plane_available(int R)
     return n > 0;
 }
 
-int loop_scheme(int R)
+static int scheme_of(const PlanChoice &pc, int R)
 {
-    const PlanChoice pc = choice_of(R);
     if (pc.scheme >= 0) return pc.scheme >= 1 && plane_available(R) ? pc.scheme : 0;
     return plane_available(R) ? 1 : 0;
+}
+
+int loop_scheme(int R) { return scheme_of(choice_of(R), R); }
+
+LoopPlan loop_plan(int R)
+{
+    const PlanChoice pc = choice_of(R);
+    return LoopPlan{{pc.v[0], pc.v[1], pc.v[2]}, scheme_of(pc, R), ztile_of(R, pc.v[2])};
 }
 
 static cudaError_t plane_variant(const LoopArgs &a, bool final_pass, int scheme, cudaStream_t s)
@@ -139,22 +131,22 @@ static cudaError_t plane_variant(const LoopArgs &a, bool final_pass, int scheme,
     return cudaErrorNotSupported;
 }
 
-cudaError_t launch_plane(const LoopArgs &a, bool final_pass, cudaStream_t s)
+cudaError_t launch_plane(const LoopPlan &p, const LoopArgs &a, bool final_pass, cudaStream_t s)
 {
-    return plane_variant(a, final_pass, loop_scheme(a.R), s);
+    return plane_variant(a, final_pass, p.scheme, s);
 }
 
-cudaError_t launch_xpass(const LoopArgs &a, bool final_pass, cudaStream_t s)
+cudaError_t launch_xpass(const LoopPlan &p, const LoopArgs &a, bool final_pass, cudaStream_t s)
 {
-    return loop_pass_variant(final_pass ? LOOP_X_FINAL : LOOP_X, choice_of(a.R).v[0], a, 0, s);
+    return loop_pass_variant(final_pass ? LOOP_X_FINAL : LOOP_X, p.v[0], a, 0, s);
 }
-cudaError_t launch_ypass(const LoopArgs &a, bool inverse, cudaStream_t s)
+cudaError_t launch_ypass(const LoopPlan &p, const LoopArgs &a, bool inverse, cudaStream_t s)
 {
-    return loop_pass_variant(inverse ? LOOP_Y_INV : LOOP_Y_FWD, choice_of(a.R).v[1], a, 0, s);
+    return loop_pass_variant(inverse ? LOOP_Y_INV : LOOP_Y_FWD, p.v[1], a, 0, s);
 }
-cudaError_t launch_zpass(const LoopArgs &a, int check_mode, cudaStream_t s)
+cudaError_t launch_zpass(const LoopPlan &p, const LoopArgs &a, int check_mode, cudaStream_t s)
 {
-    return loop_pass_variant(LOOP_Z, choice_of(a.R).v[2], a, check_mode, s);
+    return loop_pass_variant(LOOP_Z, p.v[2], a, check_mode, s);
 }
 
 // Median time (ms) of `reps` launches of one pass variant on stream s.
@@ -188,8 +180,9 @@ static cudaError_t time_variant(int kind, int v, const LoopArgs &a, int flag, cu
 }
 
 // Times every variant of every pass at volume side R on zero-filled scratch volumes
-// (the passes are data-independent in cost) and records the fastest.
-cudaError_t autotune_loop(int R, int check_mode, int *chosen, double *ms_out, int n_ms)
+// (the passes are data-independent in cost) and records the fastest; with `first`, only
+// where nothing was recorded or pinned meanwhile.
+cudaError_t autotune_loop(int R, int check_mode, bool first, int *chosen, double *ms_out, int n_ms)
 {
     const int nv = loop_plan_count(R);
     if (nv == 0) return cudaErrorInvalidValue;
@@ -325,31 +318,38 @@ cudaError_t autotune_loop(int R, int check_mode, int *chosen, double *ms_out, in
     if (e != cudaSuccess) return e;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_choice[{dev, R}] = pc;
+        if (first) g_choice.insert({{dev, R}, pc});
+        else g_choice[{dev, R}] = pc;
     }
     if (chosen)
         for (int p = 0; p < 3; p++) chosen[p] = pc.v[p];
     return cudaSuccess;
 }
 
-// Tunes R on first use on this device (see the file comment).
+static bool has_choice(int dev, int R)
+{
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    return g_choice.count({dev, R}) != 0;   // tuned or pinned
+}
+
+// Tunes R on first use on this device (see the file comment); one thread tunes, the others
+// that come meanwhile wait for its choice.
 cudaError_t ensure_tuned(int R, int check_mode, cudaStream_t s)
 {
+    static std::mutex tuning;
     const char *env = std::getenv("CTDM_AUTOTUNE");
     if (env && std::strcmp(env, "0") == 0) return cudaSuccess;
     if (loop_plan_count(R) <= 1) return cudaSuccess;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_choice.find({dev, R});
-        if (it != g_choice.end()) return cudaSuccess;   // tuned or pinned
-    }
+    if (has_choice(dev, R)) return cudaSuccess;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     e = cudaStreamIsCapturing(s, &cs);
     if (e != cudaSuccess || cs != cudaStreamCaptureStatusNone) return cudaSuccess;
-    return autotune_loop(R, check_mode, nullptr, nullptr, 0);
+    std::lock_guard<std::mutex> lk(tuning);
+    if (has_choice(dev, R)) return cudaSuccess;
+    return autotune_loop(R, check_mode, true, nullptr, nullptr, 0);
 }
 
 }  // namespace ctdm
@@ -364,7 +364,7 @@ extern "C" ctdm_status ctdm_autotune(int device, int R, int check_mode, int *var
     cudaError_t e = cudaSetDevice(device);
     if (e != cudaSuccess) return fail_cuda(e, "cudaSetDevice");
     e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = autotune_loop(R, check_mode != 0, variants3, ms, n_ms);
+    if (e == cudaSuccess) e = autotune_loop(R, check_mode != 0, false, variants3, ms, n_ms);
     if (e != cudaSuccess) return fail_cuda(e, "autotune");
     clear_error();
     return CTDM_OK;
