@@ -705,7 +705,6 @@ static ctdm_status do_positivity(ctdm_ctx *c, int R, int iters, int check_mode, 
     la.R = R;
     la.k2 = (float)k2;
     la.n_med = (float)n_med;
-    la.n_med2 = (float)(n_med * n_med);
     la.inv_r = (float)(1.0 / R);
     la.s2 = (float)(-k2 / (n_med * n_med));
     la.err = c->d_err;

@@ -350,16 +350,10 @@ struct PlanT<L_, B_, T_, Radices<FW...>, Radices<RV...>> {
     {
         stages<L, T, LP, INV, false, false, true, 1, RV...>(buf, v, tw, threadIdx.x / T, threadIdx.x % T);
     }
-    template <bool INV>
-    __device__ static __forceinline__ void run(float2 *buf, const float2 *tw)
-    {
-        float2 v[E];
-        seq<INV, true, true>(buf, v, tw);
-    }
 };
 
-// Default plan per length (2-D transforms, QPI, DCT, Ewald mapping, and variant 0
-// of the volume passes).
+// Default plan per length: variant 0 of the volume passes, and the line kernels that have no
+// plan of their own for a length (they derive theirs from this one).
 template <int L>
 struct Plan;
 #define FFTL_PLAN(LL, BB, TT, FWD, REV) \
@@ -379,12 +373,6 @@ FFTL_PLAN(1536, 8, 32, FFTL_LIST(16, 16, 3, 2), FFTL_LIST(2, 3, 16, 16))
 FFTL_PLAN(2048, 4, 64, FFTL_LIST(16, 16, 8), FFTL_LIST(8, 16, 16))
 #undef FFTL_PLAN
 #undef FFTL_LIST
-
-// First radix of the listed (forward) sequence and of the reversed one.
-template <int L>
-struct Ends {
-    static constexpr int F = Plan<L>::F0, Rv = Plan<L>::RV0;
-};
 
 // Plan variants of the volume passes, chosen per pass by the autotuner.  384 and 768 points
 // take three stages with a radix of 6 or 12 in the middle: with 4, 4, 8, 3 (8, 8, 4, 3) the
@@ -436,21 +424,6 @@ __host__ __device__ constexpr int plan_min_ctas(int want)
     // longer tiles or three-stage lengths (more twiddles live): 512
     return (P::E <= 16 && P::L <= 256) ? (want * 256 / P::THREADS > 0 ? want * 256 / P::THREADS : 1)
                                        : (P::E <= 32 ? (512 / P::THREADS > 0 ? 512 / P::THREADS : 1) : 1);
-}
-
-// Resident CTAs per SM to ask of the register allocator: `want` for register
-// tiles of up to 16 points, fewer for the longer tiles so they do not spill.
-template <int L>
-__host__ __device__ constexpr int min_ctas(int want)
-{
-    return Plan<L>::E <= 16 ? want : (Plan<L>::E <= 32 ? 2 : 1);
-}
-
-// Shared memory of the row mapping.
-template <int L>
-__host__ __device__ constexpr size_t smem_bytes_row()
-{
-    return sizeof(float2) * Plan<L>::B * (L + L / 16);
 }
 
 }  // namespace fftl

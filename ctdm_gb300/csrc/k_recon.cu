@@ -187,16 +187,6 @@ cudaError_t scale_complex(float2 *data, long n, float s, bool conjugate, cudaStr
     return cudaGetLastError();
 }
 
-cudaError_t fft3d(float2 *data, int R, bool inverse, cudaStream_t s)
-{
-    const long r2 = (long)R * R;
-    cudaError_t e = fft_rows(data, R, r2, inverse, s);
-    if (e == cudaSuccess) e = fft_cols(data, R, r2, R, r2, R, inverse, s);
-    if (e == cudaSuccess) e = fft_cols(data, R, r2, R, R, r2, inverse, s);
-    if (e == cudaSuccess && inverse) e = scale_complex(data, r2 * R, 1.0f / (float)(r2 * R), false, s);
-    return e;
-}
-
 // ------------------------------------------------------------ Ewald mapping
 // Frequency interpolation between scan angles (FrquencyInterpolation, FI_kernel and
 // calF, cTDM/Recon_kernel.cu:471-731, with the mathematics fixed).  A frame puts its

@@ -97,7 +97,7 @@ struct LoopArgs {
     const uint8_t *mask;
     float2 *out;            // final RI volume (octant shifted), only for the final pass
     int R;
-    float k2, n_med, n_med2;
+    float k2, n_med;
     // -1 / (S k^2) with S what the inverse transforms leave unnormalised: R^3, or where
     // empty tiles are skipped R^2 on the plane scheme and R on the line passes
     float s1;
@@ -245,8 +245,6 @@ cudaError_t fft_rows_from(const float2 *src, float2 *dst, int L, long nlines, bo
                           cudaStream_t s);
 cudaError_t fft_cols_from(const float2 *src, float2 *dst, int L, long nlines, int nx, long plane, long ld,
                           bool inverse, float scale, cudaStream_t s, const int *xactive = nullptr);
-// 3-D transform in place (cuFFT3D semantics: inverse scaled by 1/(R^3)).
-cudaError_t fft3d(float2 *data, int R, bool inverse, cudaStream_t s);
 cudaError_t scale_complex(float2 *data, long n, float s, bool conjugate, cudaStream_t st);
 
 }  // namespace ctdm

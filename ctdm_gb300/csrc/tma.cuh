@@ -91,40 +91,6 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
                  : "memory");
 }
 
-// Contiguous bulk copy shared -> global in the calling thread's bulk group.  The
-// writers of the shared source run fence_async_smem() and a barrier first.
-__device__ __forceinline__ void bulk_store(void *dst, const void *src, uint32_t bytes)
-{
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
-                     static_cast<uint64_t>(__cvta_generic_to_global(dst))),
-                 "r"(smem_addr(src)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Waits until every committed bulk store has finished reading shared memory.
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// Makes this thread's generic-proxy shared-memory writes visible to bulk copies.
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// Distributed shared memory: the shared::cluster address of `p` (an address in this
-// CTA's shared memory) in the CTA of cluster rank `rank`, and 64-bit accesses to it.
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t local_smem_addr, uint32_t rank)
-{
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ float2 ld_cluster(uint32_t addr)
-{
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, float2 v)
-{
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
-}
-
 // Prefetch a tensor map descriptor (a kernel parameter) into the descriptor cache.
 __device__ __forceinline__ void prefetch_map(const CUtensorMap *map)
 {

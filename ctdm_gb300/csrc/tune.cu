@@ -241,7 +241,6 @@ cudaError_t autotune_loop(int R, int check_mode, bool first, int *chosen, double
         a.inv_r = (float)(1.0 / R);
         a.k2 = (float)k2;
         a.n_med = (float)nm;
-        a.n_med2 = (float)(nm * nm);
         a.s1 = (float)(-1.0 / ((double)r3 * k2));
         a.s2 = (float)(-k2 / (nm * nm));
         a.err = err;
