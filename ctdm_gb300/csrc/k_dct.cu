@@ -112,13 +112,25 @@ __device__ __forceinline__ int dct_pos(int i, int t)
     return dct_upper<M, T, R>(i, t) ? 2 * (M - 1 - n) + 1 : 2 * n;
 }
 
-// DCT-II coefficients k of the two real lines packed in Z: z = Z[k], r = Z[-k], w the
-// coefficient's (cos, sin)(pi k / 2M); scale dT, and dT / sqrt 2 for k = 0 (countFDCT :202-216).
-__device__ __forceinline__ float2 dct_pair(float2 z, float2 r, float2 w, float scale)
+// DCT-II coefficients k of the two real lines packed in Z, unscaled: z = Z[k], r = Z[-k], w the
+// coefficient's (cos, sin)(pi k / 2M).  The reference scales every coefficient by 1 / sqrt(2M)
+// forward and back, k = 0 by 1 / sqrt 2 less and more (countFDCT :202-216, countIDCT :218-246):
+// 1 / (2M)^2 over the four transforms, applied once, where it is exact for a power of two.
+__device__ __forceinline__ float2 dct_pair(float2 z, float2 r, float2 w)
 {
-    return make_float2(scale * ((z.x + r.x) * w.x + (z.y - r.y) * w.y),
-                       scale * ((z.y + r.y) * w.x - (z.x - r.x) * w.y));
+    return make_float2((z.x + r.x) * w.x + (z.y - r.y) * w.y, (z.y + r.y) * w.x - (z.x - r.x) * w.y);
 }
+
+// Sum with the rounding errors of its additions beside it (Knuth's two-sum); x + lo is added.
+struct Sum2 {
+    float s = 0.f, e = 0.f;
+    __device__ __forceinline__ void add(float x, float lo)
+    {
+        const float t = __fadd_rn(s, x), z = __fsub_rn(t, s);
+        e = __fadd_rn(e, __fadd_rn(lo, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z))));
+        s = t;
+    }
+};
 
 // phi, T, out: A maps of M x M (T: scratch).  dtw[k] = (cos, sin)(k pi / 2M), tw: M-point
 // twiddles, mir = (1 + cos phi, sin phi).
@@ -140,7 +152,7 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
     const int rank = (int)(blockIdx.x % C);   // the cluster rank when a cluster takes the map
     const long map = (long)(blockIdx.x / C) * M * M;
     const int tid = threadIdx.x;
-    const float dT = 1.0f / sqrtf(2.0f * M), dT0 = dT * 0.70710678118654752440f;
+    const float inv0 = 1.0f / mir.x;   // k = 0 counts once in the inverse's f(n)
 
     // ---- rows: Laplacian and DCT-II, two rows per complex line
     if constexpr (PHASE == DCT_ALL || PHASE == DCT_ROWS) {
@@ -174,8 +186,42 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
                 }
             }
             __syncthreads();
+            // Coefficient k = 1 from a sum of its own (eights by a tree, those compensated) above 256: the divide weights the
+            // lowest coefficients most, and the M-point transform rounds them more than the
+            // 2M-point one of the mirrored line did.  Error of the unwrapped phase, relative L2
+            // over 192 noisy maps, that form / without the sum / with it: 4.5 / 4.9 / 4.1e-7 at 384,
+            // 5.6 / 6.4 / 5.4 at 512, 9.0 / 10.0 / 7.9 at 768; up to 256 no larger as it is.  121 of
+            // 512^2: 400 -> 404 us.
+            Sum2 c1a, c1b;
             float2 v[E];
-            P::template seq_row_from<false>(buf, v, tws);
+            if constexpr (M > 256) {
+#pragma unroll
+                for (int i = 0; i < E; i++) v[i] = line[Y::at(fftl::slot_pos<M, P::T, P::F0>(i, t))];
+                __syncthreads();   // the transform's exchanges write the lines
+#pragma unroll
+                for (int i0 = 0; i0 < E; i0 += 8) {
+                    float2 p[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        const int n = fftl::slot_pos<M, P::T, P::F0>(i0 + i, t);
+                        p[i] = cscale(v[i0 + i], __ldg(&dts[n < M / 2 ? 4 * n + 1 : 4 * (M - 1 - n) + 3]).x);
+                    }
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+                        for (int i = 0; i < o; i++) p[i] = cadd(p[i], p[i + o]);
+                    c1a.add(p[0].x, 0.f);
+                    c1b.add(p[0].y, 0.f);
+                }
+#pragma unroll
+                for (int o = P::T / 2; o > 0; o >>= 1) {
+                    c1a.add(__shfl_xor_sync(0xffffffffu, c1a.s, o), __shfl_xor_sync(0xffffffffu, c1a.e, o));
+                    c1b.add(__shfl_xor_sync(0xffffffffu, c1b.s, o), __shfl_xor_sync(0xffffffffu, c1b.e, o));
+                }
+                P::template seq_row<false>(buf, v, tws);
+            } else {
+                P::template seq_row_from<false>(buf, v, tws);
+            }
             __syncwarp();
 #pragma unroll
             for (int i = 0; i < E; i++) line[Y::at(fftl::slot_pos<M, P::T, P::RV0>(i, t))] = v[i];
@@ -184,7 +230,9 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
 #pragma unroll
             for (int i = 0; i < E; i++) {
                 const int k = fftl::slot_pos<M, P::T, P::RV0>(i, t);
-                const float2 x = dct_pair(v[i], line[Y::at(k == 0 ? 0 : M - k)], __ldg(&dts[k]), k == 0 ? dT0 : dT);
+                float2 x = dct_pair(v[i], line[Y::at(k == 0 ? 0 : M - k)], __ldg(&dts[k]));
+                if (M > 256 && k == 1)
+                    x = make_float2(2.f * __fadd_rn(c1a.s, c1a.e), 2.f * __fadd_rn(c1b.s, c1b.e));
                 __stcg(&row[k], x.x);
                 __stcg(&row[M + k], x.y);
             }
@@ -218,13 +266,13 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
 #pragma unroll
             for (int i = 0; i < E; i++) {
                 const int k = fftl::slot_pos<M, P::T, P::RV0>(i, t);
-                float2 x = dct_pair(v[i], line[k == 0 ? 0 : M - k], __ldg(&dts[k]), k == 0 ? dT0 : dT);
+                float2 x = dct_pair(v[i], line[k == 0 ? 0 : M - k], __ldg(&dts[k]));
                 // devConstant (:300-311): / (2cos(4 pi i/(4M-1)) + 2cos(4 pi j/(4M-1)) - 4), (0,0) -> 0;
                 // the denominator is -(4 sin^2(2 pi i/(4M-1)) + 4 sin^2(2 pi j/(4M-1))), free of cancellation
                 const float ey = __ldg(&egs[k]);
                 x.x = kx == 0 && k == 0 ? 0.f : x.x / (-(exa + ey));
                 x.y = x.y / (-(exb + ey));
-                const float s = k == 0 ? dT * 1.41421356237309504880f / mir.x : dT;
+                const float s = (k == 0 ? inv0 : 1.0f) * (1.0f / (4.0f * M * M));
                 S[k * P::B + b] = x.y * s;
                 xa[i] = x.x * s;
             }
@@ -261,8 +309,8 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
 #pragma unroll
             for (int i = 0; i < E; i++) {
                 const int k = fftl::slot_pos<M, P::T, P::F0>(i, t);
-                const float s = k == 0 ? dT * 1.41421356237309504880f / mir.x : dT;
-                v[i] = cscale(__ldg(&dts[k]), s * __ldcg(&T[row + k]));
+                const float x = __ldcg(&T[row + k]);
+                v[i] = cscale(__ldg(&dts[k]), k == 0 ? inv0 * x : x);
             }
             __syncwarp();
             P::template seq_row<true>(buf, v, tws);
