@@ -21,6 +21,7 @@
 //   f(n) = Y_0 + Re((1 + e^(-i phi)) (W(n) - Y_0)),
 // W at even n is IFFT_M(Y), and W(2M - 1 - n) = conj W(n) gives the odd n from it: one
 // M-point transform per line for either mode.
+#include <climits>
 #include <cmath>
 
 #include <cooperative_groups.h>
@@ -36,27 +37,33 @@ namespace ctdm {
 // 16 rows per CTA (32 at 256), so that the phases' loads, barriers and tails are paid once;
 // larger maps would leave a cluster of 8 several steps in a row (512^2: 109 us for one map
 // against 45 for three launches), so there each phase is a launch over all steps.
-// Measured against three launches of 2M-point transforms: one 128^2 map 38.9 -> 16.0 us,
-// 121 of 256^2 184 -> 104 us (38% issue active, 26 warps per SM: latency of the phases'
+// Measured against three launches of 2M-point transforms: one 128^2 map 38.9 -> 13.0 us,
+// 121 of 256^2 184 -> 103 us (38% issue active, 26 warps per SM: latency of the phases'
 // chains and barriers; 19 us for the maps' bytes at the copy peak), 16 of 768^2 527 ->
-// 190 us.  64 registers at 256 spill 330 bytes a thread and still beat 80 (117 us): with 3
-// CTAs per SM the 121 clusters take three waves instead of two.
+// 190 us.  64 registers at 256 spill 330 bytes a thread and still beat 80 (117 us for the 121
+// maps): with 3 CTAs per SM their clusters take three waves instead of two.
+// CHAIN: maps up to which the launch is chained.  Clusters placed while the kernel before still
+// holds most SMs crowd together on the first ones that are free: 256^2 chained against not,
+// 29.3 / 31.8 us for one map, 29.9 / 32.7 for 9, 43.1 / 32.8 for 10, 52.6 / 37.8 for 16, 110 / 103
+// for 121; 128^2 13.0 / 15.8 for one, 14.6 / 16.4 for 13, 19.9 / 16.4 for 14; 64^2 12.6 / 14.4 for
+// 32, 15.8 / 14.4 for 40.  Clusters of one or two CTAs and the three launches of the larger
+// maps gain at any count (121 of 32^2 12.0 / 14.4, 16 of 512^2 75.6 / 81.7).
 template <int M>
 struct DctCfg;
-#define CTDM_DCT(MM, CC, OCC, ...)                            \
+#define CTDM_DCT(MM, CC, OCC, CH, ...)                        \
     template <>                                               \
     struct DctCfg<MM> {                                       \
-        static constexpr int C = CC, RESIDENT = OCC;          \
+        static constexpr int C = CC, RESIDENT = OCC, CHAIN = CH;  \
         using P = __VA_ARGS__;                                \
     };
-CTDM_DCT(16, 1, 768, fftl::PlanT<16, 8, 4, fftl::Radices<4, 4>, fftl::Radices<4, 4>>)
-CTDM_DCT(32, 2, 768, fftl::PlanT<32, 8, 4, fftl::Radices<8, 4>, fftl::Radices<4, 8>>)
-CTDM_DCT(64, 4, 768, fftl::PlanT<64, 8, 8, fftl::Radices<8, 8>, fftl::Radices<8, 8>>)
-CTDM_DCT(128, 8, 768, fftl::PlanT<128, 8, 16, fftl::Radices<8, 4, 4>, fftl::Radices<4, 4, 8>>)
-CTDM_DCT(256, 8, 1024, fftl::Plan<256>)
-CTDM_DCT(384, 24, 512, fftl::PV<384, 2>)
-CTDM_DCT(512, 32, 768, fftl::PV<512, 2>)
-CTDM_DCT(768, 48, 512, fftl::PV<768, 1>)
+CTDM_DCT(16, 1, 768, INT_MAX, fftl::PlanT<16, 8, 4, fftl::Radices<4, 4>, fftl::Radices<4, 4>>)
+CTDM_DCT(32, 2, 768, INT_MAX, fftl::PlanT<32, 8, 4, fftl::Radices<8, 4>, fftl::Radices<4, 8>>)
+CTDM_DCT(64, 4, 768, 32, fftl::PlanT<64, 8, 8, fftl::Radices<8, 8>, fftl::Radices<8, 8>>)
+CTDM_DCT(128, 8, 768, 13, fftl::PlanT<128, 8, 16, fftl::Radices<8, 4, 4>, fftl::Radices<4, 4, 8>>)
+CTDM_DCT(256, 8, 1024, 9, fftl::Plan<256>)
+CTDM_DCT(384, 24, 512, INT_MAX, fftl::PV<384, 2>)
+CTDM_DCT(512, 32, 768, INT_MAX, fftl::PV<512, 2>)
+CTDM_DCT(768, 48, 512, INT_MAX, fftl::PV<768, 1>)
 #undef CTDM_DCT
 enum DctPhase { DCT_ALL = 0, DCT_ROWS = 1, DCT_COLS = 2, DCT_ROWS_INV = 3 };
 
@@ -349,8 +356,9 @@ static cudaError_t dct_phase(const float *phi, float *out, float *T, int A, int 
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // chained (chain_begin)
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    // chained (chain_begin) up to CHAIN maps
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = A <= DctCfg<M>::CHAIN ? 1 : 0;
     attr[1].id = cudaLaunchAttributeClusterDimension;
     attr[1].val.clusterDim.x = C;
     attr[1].val.clusterDim.y = 1;

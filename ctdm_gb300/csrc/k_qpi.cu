@@ -363,8 +363,14 @@ static cudaError_t qpi_rows_launch(const float *bg, int nbg, const T *holo, int 
     const long bgpairs = (long)nbg * N / 2, npairs = bgpairs + (long)A * N / 2;
     cudaError_t e = set_smem<N>(qpi_rows_kernel<N, T>, smem_r);
     if (e != cudaSuccess) return e;
-    return launch_chained(qpi_rows_kernel<N, T>, dim3((unsigned)((npairs + PR::B - 1) / PR::B)), dim3(PR::THREADS),
-                          smem_r, s, bg, holo, T1, carrier, bgpairs, npairs, M, twiddles(N));
+    // Chained up to one wave.  CTAs that start before the SMs have drained run with the split of
+    // L1 and shared memory of the kernel before (the carrier search prefers shared memory), and
+    // an SM that is never empty keeps it: Algorithm A on 61 x 1024^2 holograms 230 us chained,
+    // 214 not, 61 x 2048^2 1057 and 960, 8 x 1024^2 (1.7 waves) 94 and 91.
+    const long grid = (npairs + PR::B - 1) / PR::B;
+    const bool chain = grid <= wave_ctas(qpi_rows_kernel<N, T>, PR::THREADS, smem_r);
+    return launch_chained_if(chain, qpi_rows_kernel<N, T>, dim3((unsigned)grid), dim3(PR::THREADS), smem_r, s, bg, holo,
+                             T1, carrier, bgpairs, npairs, M, twiddles(N));
 }
 
 template <int N>
@@ -456,8 +462,8 @@ __device__ __forceinline__ float qpib_tap(const float *__restrict__ h, int N, fl
     return b * t2 + (-t1 * b + t1);
 }
 
-// holo: A holograms N x N; pairs q cover output rows (2q, 2q+1) of the A * N/4 rows.
-// Images: nbg of bg, then holograms of holo; image k's row pairs are the k-th N/8.
+// Images N x N: nbg of bg, then those of holo.  Pair q covers output rows (2q, 2q+1) of all
+// images' N/4 rows each, so image k's pairs are the k-th N/8.
 // mag != NULL: |X| of the shifted spectrum rows (N floats per row).  Else T gets
 // the M = N/4 window columns per row, half-swapped, around center[1] for the first of holo's
 // images and center[0] for the others.
@@ -480,7 +486,7 @@ __global__ void __launch_bounds__(QRows<N>::THREADS) qpib_rows_kernel(const floa
     const int t = threadIdx.x % P::T, b = threadIdx.x / P::T;
     const long q = (long)blockIdx.x * P::B + b;
     const bool ok = q < npairs;
-    const long r0 = ok ? 2 * q : 0;                 // global output row (a * H + j)
+    const long r0 = ok ? 2 * q : 0;                 // global output row (image * H + j)
     const int img = (int)(r0 / H);                  // H is even: both rows of one image
     const float *h0 = img < nbg ? bg + (long)img * N * N : holo + (long)(img - nbg) * N * N;
     const int j0 = (int)(r0 % H), j1 = j0 + 1;

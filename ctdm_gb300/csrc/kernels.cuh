@@ -42,8 +42,10 @@ __device__ __forceinline__ void chain_begin()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
+// chain = false: an ordinary launch, which starts on drained SMs (chain_begin returns at once).
 template <class... KA, class... A>
-cudaError_t launch_chained(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+cudaError_t launch_chained_if(bool chain, void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                              A... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -54,10 +56,15 @@ cudaError_t launch_chained(void (*kernel)(KA...), dim3 grid, dim3 block, size_t 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chain ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(args)...);
     note_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+template <class... KA, class... A>
+cudaError_t launch_chained(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+    return launch_chained_if(true, kernel, grid, block, smem, s, args...);
 }
 
 // ---- per-angle Ewald geometry (host computed, FP64 rule inputs)
