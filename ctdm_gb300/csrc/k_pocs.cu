@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(P::THREADS, row_min_ctas<P>())
 // octant shifted like cuFFT3Dshift.
 template <int L>
 struct StoreIndex {
+    static constexpr bool READS = false;
     float2 *ri;
     float inv_r, n_med;
     __device__ __forceinline__ void operator()(long i, float2 v) const

@@ -30,6 +30,8 @@ __host__ __device__ constexpr int row_min_ctas()
 // stages.  HBM-bound: at 256^3 complex to complex, in place, 59.9 -> 47 us per launch
 // against the form that staged whole lines in shared memory between CTA barriers (40 us
 // at the copy peak); 181 x 512 rows of 512, 193 -> 146 us.
+// A storer that reads what it overwrites (READS) takes a thread's points together: point by
+// point each load would wait for the store before it.
 template <class P, bool INV, class LD, class ST>
 __global__ void __launch_bounds__(P::THREADS, row_min_ctas<P>())
     rows_fn_kernel(LD ld, ST st, const float2 *__restrict__ tw, long nlines)
@@ -47,10 +49,16 @@ __global__ void __launch_bounds__(P::THREADS, row_min_ctas<P>())
 #pragma unroll
     for (int i = 0; i < P::E; i++)
         v[i] = ok ? ld(base + fftl::slot_pos<L, P::T, P::F0>(i, t)) : make_float2(0.f, 0.f);
+    if constexpr (ST::READS)
+        if (ok) st.template begin<P>(base, t);
     P::template seq_row<INV>(buf, v, tw);
     if (!ok) return;
+    if constexpr (ST::READS) {
+        st.template row<P>(base, t, v);
+    } else {
 #pragma unroll
-    for (int i = 0; i < P::E; i++) st(base + fftl::slot_pos<L, P::T, P::RV0>(i, t), v[i]);
+        for (int i = 0; i < P::E; i++) st(base + fftl::slot_pos<L, P::T, P::RV0>(i, t), v[i]);
+    }
 }
 
 // Once per kernel and device: the shared-memory opt-in and the largest carveout.
@@ -125,6 +133,7 @@ struct LoadComplex {
     __device__ __forceinline__ float2 operator()(long i) const { return __ldcs(p + i); }
 };
 struct StoreScaled {
+    static constexpr bool READS = false;
     float2 *p;
     float scale;
     __device__ __forceinline__ void operator()(long i, float2 v) const { __stcs(p + i, cscale(v, scale)); }
