@@ -580,14 +580,8 @@ __global__ void __launch_bounds__(1024) qpib_center_kernel(const float *__restri
 // Inverse M-point transforms of the window rows, 1/M, conjugate, transposed store:
 // field[a][X * M + Y] from row Y, column X (polar: as argument and modulus); with bgf the
 // phase / amplitude epilogue of calcWrapPhase instead (cTDM/HilbertTransform.cu:3618-3639).
-// 16 lines per CTA at M = 128 (twice the CTAs of the default plan): a scan of 49 frames of
-// 128 rows leaves a third of the SMs a second CTA of 32.
 template <int M>
-struct QbInv : Plan<M> {};
-template <> struct QbInv<128> : fftl::PlanT<128, 16, 8, fftl::Radices<16, 8>, fftl::Radices<8, 16>> {};
-
-template <int M>
-__global__ void __launch_bounds__(QbInv<M>::THREADS) qpib_inv_kernel(const float2 *__restrict__ T, long nrows,
+__global__ void __launch_bounds__(Plan<M>::THREADS) qpib_inv_kernel(const float2 *__restrict__ T, long nrows,
                                                                     float2 *field_out, bool polar,
                                                                     const float2 *__restrict__ bgf, long bg_stride,
                                                                     float *phase, float *amp,
@@ -596,7 +590,7 @@ __global__ void __launch_bounds__(QbInv<M>::THREADS) qpib_inv_kernel(const float
     chain_begin();
     T = fresh(T);
     bgf = fresh(bgf);
-    using P = QbInv<M>;
+    using P = Plan<M>;
     extern __shared__ float4 smem4[];
     float2 *buf = reinterpret_cast<float2 *>(smem4);
     const long row0 = (long)blockIdx.x * P::B;
@@ -651,7 +645,7 @@ template <int M>
 static cudaError_t qpib_inv_launch(const float2 *T, int A, float2 *field_out, bool polar, const float2 *bgf,
                                    long bg_stride, float *phase, float *amp, cudaStream_t s)
 {
-    using P = QbInv<M>;
+    using P = Plan<M>;
     const size_t smem = fftl::plan_smem<P>();
     cudaError_t e = set_smem<M>(qpib_inv_kernel<M>, smem);
     if (e != cudaSuccess) return e;
