@@ -30,6 +30,7 @@ using namespace ctdm;
 struct ctdm_tape {
     int device = 0, R = 0, TB = 0;
     long S = 0, tiles = 0;
+    void *base = nullptr;      // the allocation of the arrays up to red
     uint32_t *idx = nullptr;   // S voxel indices, ascending
     float2 *y = nullptr;       // S data values (scaled by 1 / (-k^2 R^{3/2}))
     float2 *work = nullptr;    // R^3 transform buffer
@@ -728,19 +729,17 @@ extern "C" ctdm_status ctdm_tape_create(int device, int R, const ctdm_cfloat *d_
     t->TB = tile_lines(R);
     t->tiles = (long)R * R / t->TB;
     const long tv = (long)tv_tiles(R) * ((R + 3) / 4), parts = t->tiles > tv ? t->tiles : tv;
-    uint8_t *flags = nullptr;   // measured voxels, while the tape is built
-    int *bc = nullptr;          // block counts, then offsets
+    // while the tape is built: block counts, then offsets; measured voxels
     struct Scratch {
-        uint8_t *&f;
-        int *&b;
+        void *p = nullptr;
         ~Scratch()
         {
-            if (f) cudaFree(f);
-            if (b) cudaFree(b);
+            if (p) cudaFree(p);
         }
-    } scratch{flags, bc};
-    if ((e = cudaMalloc(&flags, n)) != cudaSuccess || (e = cudaMalloc(&bc, sizeof(int) * 2 * nb)) != cudaSuccess)
-        return cleanup(cuda_fail(e, "alloc"));
+    } scratch;
+    if ((e = cudaMalloc(&scratch.p, sizeof(int) * 2 * nb + n)) != cudaSuccess) return cleanup(cuda_fail(e, "alloc"));
+    int *bc = static_cast<int *>(scratch.p);
+    uint8_t *flags = reinterpret_cast<uint8_t *>(bc + 2 * nb);
     measured_flags<<<grid_for(n), 256>>>(reinterpret_cast<const float2 *>(d_F2), d_counts, n, flags); note_launch();
     block_counts<<<nb, kScanBlock>>>(flags, n, chunk, bc); note_launch();
     std::vector<int> hc(nb), ho(nb);
@@ -754,19 +753,33 @@ extern "C" ctdm_status ctdm_tape_create(int device, int R, const ctdm_cfloat *d_
     t->S = S;
     if (S == 0) return cleanup(fail(CTDM_ERR_INVALID, "ctdm_tape_create: no measured voxels%s"));
     const size_t rows = (size_t)t->tiles * R;
-    if ((e = cudaMemcpy(bc + nb, ho.data(), sizeof(int) * nb, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = cudaMalloc(&t->idx, sizeof(uint32_t) * S)) != cudaSuccess ||
-        (e = cudaMalloc(&t->y, sizeof(float2) * S)) != cudaSuccess ||
-        (e = cudaMalloc(&t->work, sizeof(float2) * n)) != cudaSuccess ||
-        (e = cudaMalloc(&t->tmask, sizeof(uint32_t) * rows)) != cudaSuccess ||
-        (e = cudaMalloc(&t->tprefix, sizeof(int) * rows)) != cudaSuccess ||
-        (e = cudaMalloc(&t->tcount, sizeof(int) * t->tiles)) != cudaSuccess ||
-        (e = cudaMalloc(&t->toff, sizeof(int) * t->tiles)) != cudaSuccess ||
-        (e = cudaMalloc(&t->active, sizeof(int) * active_ints(R))) != cudaSuccess ||
-        (e = cudaMalloc(&t->rank, sizeof(int) * S)) != cudaSuccess ||
-        (e = cudaMalloc(&t->yt, sizeof(float2) * S)) != cudaSuccess ||
-        (e = cudaMalloc(&t->red, sizeof(double) * (parts + 1))) != cudaSuccess)
+    // the tape's arrays share one allocation
+    size_t bytes = 0;
+    auto place = [&](size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) & ~(size_t)255;
+        return at;
+    };
+    const size_t o_work = place(sizeof(float2) * n), o_idx = place(sizeof(uint32_t) * S), o_y = place(sizeof(float2) * S),
+                 o_mask = place(sizeof(uint32_t) * rows), o_pre = place(sizeof(int) * rows),
+                 o_cnt = place(sizeof(int) * t->tiles), o_off = place(sizeof(int) * t->tiles),
+                 o_act = place(sizeof(int) * active_ints(R)), o_rank = place(sizeof(int) * S),
+                 o_yt = place(sizeof(float2) * S), o_red = place(sizeof(double) * (parts + 1));
+    if ((e = cudaMemcpyAsync(bc + nb, ho.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, 0)) != cudaSuccess ||
+        (e = cudaMalloc(&t->base, bytes)) != cudaSuccess)
         return cleanup(cuda_fail(e, "alloc"));
+    char *base = static_cast<char *>(t->base);
+    t->work = reinterpret_cast<float2 *>(base + o_work);
+    t->idx = reinterpret_cast<uint32_t *>(base + o_idx);
+    t->y = reinterpret_cast<float2 *>(base + o_y);
+    t->tmask = reinterpret_cast<uint32_t *>(base + o_mask);
+    t->tprefix = reinterpret_cast<int *>(base + o_pre);
+    t->tcount = reinterpret_cast<int *>(base + o_cnt);
+    t->toff = reinterpret_cast<int *>(base + o_off);
+    t->active = reinterpret_cast<int *>(base + o_act);
+    t->rank = reinterpret_cast<int *>(base + o_rank);
+    t->yt = reinterpret_cast<float2 *>(base + o_yt);
+    t->red = reinterpret_cast<double *>(base + o_red);
     const float scale = (float)(1.0 / (-k2 * std::pow((double)R, 1.5)));
     block_write<<<nb, kScanBlock>>>(flags, bc + nb, n, chunk, reinterpret_cast<const float2 *>(d_F2), scale, t->idx,
                                     t->y); note_launch();
@@ -787,9 +800,7 @@ extern "C" void ctdm_tape_destroy(ctdm_tape *t)
 {
     if (!t) return;
     cudaSetDevice(t->device);
-    for (void *p : {(void *)t->idx, (void *)t->y, (void *)t->work, (void *)t->tmask, (void *)t->tprefix,
-                    (void *)t->tcount, (void *)t->toff, (void *)t->active, (void *)t->rank, (void *)t->yt,
-                    (void *)t->wmom, (void *)t->wmom2, (void *)t->grad, (void *)t->red})
+    for (void *p : {t->base, (void *)t->wmom, (void *)t->wmom2, (void *)t->grad})
         if (p) cudaFree(p);
     delete t;
 }
