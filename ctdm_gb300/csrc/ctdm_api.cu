@@ -1759,7 +1759,7 @@ extern "C" void extractQPI_AlgorithmA(ctdm_cfloat *SP, ctdm_cfloat *BG, ctdm_cfl
     if (e == cudaSuccess) e = cudaMemcpy(stage, SP, sizeof(float2) * nn, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = real_parts(stage, B<float>(c, B_HOLO), nn, 0);
     if (e != cudaSuccess) { cuda_fail(e, "extractQPI_AlgorithmA upload"); return; }
-    // carrier (detected from the background on frame 1) and the background field
+    // carrier (detected from the background on frame 1) and the buffers
     if (qpi_setup(c, N, M, 1, B<float>(c, B_BG), 0, known, 0) != CTDM_OK) return;
     if (frame == 1) {
         int host[3] = {0, 0, 0};

@@ -40,8 +40,10 @@ namespace ctdm {
 // Measured against three launches of 2M-point transforms: one 128^2 map 38.9 -> 13.0 us,
 // 121 of 256^2 184 -> 103 us (38% issue active, 26 warps per SM: latency of the phases'
 // chains and barriers; 19 us for the maps' bytes at the copy peak), 16 of 768^2 527 ->
-// 190 us.  64 registers at 256 spill 330 bytes a thread and still beat 80 (117 us for the 121
-// maps): with 3 CTAs per SM their clusters take three waves instead of two.
+// 190 us.  64 registers at 256 spill 340 bytes a thread and still beat 80 for scans of 121, 181
+// and 242 maps (103 / 113, 154 / 159, 198 / 203 us): with 3 CTAs per SM the 121 clusters take three
+// waves instead of two.  Between and below, 80 would be the faster (16 maps 37.8 / 34.8, 49 49.3 /
+// 44.6, 150 136 / 128).
 // CHAIN: maps up to which the launch is chained.  Clusters placed while the kernel before still
 // holds most SMs crowd together on the first ones that are free: 256^2 chained against not,
 // 29.3 / 31.8 us for one map, 29.9 / 32.7 for 9, 43.1 / 32.8 for 10, 52.6 / 37.8 for 16, 110 / 103

@@ -337,6 +337,11 @@ __global__ void __launch_bounds__(kThreads, 3) tv_kernel(const float *__restrict
     fetch(z1, la, lb);
     take(la, lb, c);
     fetch(z1 - 1, la, lb);
+    // |g|^2 of the thread's voxels (148 at 256^3, 512 at 384^3) in float, the threads' sums in
+    // double: the roundings add up to about 1e-9 of the norm over 1e5 threads.  Double every 16
+    // planes cost the step 11% from shared memory and 23% from registers (the next plane's loads
+    // stay behind the branch), a compensated float sum 21% (spills); the volume's error against
+    // 64 bits was the same.
     float acc = 0.f;
     // plane z1 only gives q_z
     for (int z = z1; z >= z0; z--) {

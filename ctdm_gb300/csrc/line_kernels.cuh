@@ -11,7 +11,8 @@
 namespace ctdm {
 
 // Plan of the row kernels: 16 or 24 points per thread where the length allows, and at
-// most 32 threads per line, so that a line's exchanges need warp barriers only.
+// most 32 threads per line, so that a line's exchanges need warp barriers only (64 threads at
+// 2048 points, with a named barrier per line).
 template <int L>
 struct RowPlan : fftl::Plan<L> {};
 template <> struct RowPlan<384> : fftl::PV<384, 1> {};
