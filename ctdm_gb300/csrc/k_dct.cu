@@ -37,11 +37,11 @@ namespace ctdm {
 // 16 rows per CTA (32 at 256), so that the phases' loads, barriers and tails are paid once;
 // larger maps would leave a cluster of 8 several steps in a row (512^2: 109 us for one map
 // against 45 for three launches), so there each phase is a launch over all steps.
-// Measured against three launches of 2M-point transforms: one 128^2 map 38.9 -> 13.0 us,
-// 121 of 256^2 184 -> 103 us (38% issue active, 26 warps per SM: latency of the phases'
+// Measured against three launches of 2M-point transforms: one 128^2 map 38.9 -> 13.3 us,
+// 121 of 256^2 184 -> 106 us (38% issue active, 26 warps per SM: latency of the phases'
 // chains and barriers; 19 us for the maps' bytes at the copy peak), 16 of 768^2 527 ->
 // 190 us.  64 registers at 256 spill 340 bytes a thread and still beat 80 for scans of 121, 181
-// and 242 maps (103 / 113, 154 / 159, 198 / 203 us): with 3 CTAs per SM the 121 clusters take three
+// and 242 maps (103 / 113, 154 / 159, 198 / 203 us without the sum of k = 1): with 3 CTAs per SM the 121 clusters take three
 // waves instead of two.  Between and below, 80 would be the faster (16 maps 37.8 / 34.8, 49 49.3 /
 // 44.6, 150 136 / 128).
 // CHAIN: maps up to which the launch is chained.  Clusters placed while the kernel before still
@@ -195,15 +195,18 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
                 }
             }
             __syncthreads();
-            // Coefficient k = 1 from a sum of its own (eights by a tree, those compensated) above 256: the divide weights the
-            // lowest coefficients most, and the M-point transform rounds them more than the
-            // 2M-point one of the mirrored line did.  Error of the unwrapped phase, relative L2
-            // over 192 noisy maps, that form / without the sum / with it: 4.5 / 4.9 / 4.1e-7 at 384,
-            // 5.6 / 6.4 / 5.4 at 512, 9.0 / 10.0 / 7.9 at 768; up to 256 no larger as it is.  121 of
-            // 512^2: 400 -> 404 us.
+            // Coefficient k = 1 from a sum of its own (eights by a tree, those compensated): the divide
+            // weights the lowest coefficients most, and the M-point transform rounds them more than
+            // the 2M-point one of the mirrored line did.  Error of the unwrapped phase, relative L2
+            // over 192 maps of a specimen, that form / without the sum / with it: 2.5 / 1.8 / 1.7e-7
+            // at 64, 2.2 / 2.2 / 2.0 at 128, 3.2 / 3.2 / 2.9 at 256, 4.5 / 4.9 / 4.1 at 384, 5.6 / 6.4 / 5.4
+            // at 512, 9.0 / 10.0 / 7.9 at 768; over 320 maps of noise 2.2 / 2.3 / 2.0e-6 at 64, 4.0 / 4.5 /
+            // 3.9 at 128, 8.6 / 9.3 / 8.2 at 256 (16 needs none).  One map of 128^2 13.0 -> 13.3 us, 121
+            // of 256^2 103.7 -> 105.7, of 512^2 400 -> 404.
+            constexpr bool APART = M >= 32;
             Sum2 c1a, c1b;
             float2 v[E];
-            if constexpr (M > 256) {
+            if constexpr (APART) {
 #pragma unroll
                 for (int i = 0; i < E; i++) v[i] = line[Y::at(fftl::slot_pos<M, P::T, P::F0>(i, t))];
                 __syncthreads();   // the transform's exchanges write the lines
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
             for (int i = 0; i < E; i++) {
                 const int k = fftl::slot_pos<M, P::T, P::RV0>(i, t);
                 float2 x = dct_pair(v[i], line[Y::at(k == 0 ? 0 : M - k)], __ldg(&dts[k]));
-                if (M > 256 && k == 1)
+                if (APART && k == 1)
                     x = make_float2(2.f * __fadd_rn(c1a.s, c1a.e), 2.f * __fadd_rn(c1b.s, c1b.e));
                 __stcg(&row[k], x.x);
                 __stcg(&row[M + k], x.y);
