@@ -37,7 +37,7 @@ namespace ctdm {
 // 16 rows per CTA (32 at 256), so that the phases' loads, barriers and tails are paid once;
 // larger maps would leave a cluster of 8 several steps in a row (512^2: 109 us for one map
 // against 45 for three launches), so there each phase is a launch over all steps.
-// Measured against three launches of 2M-point transforms: one 128^2 map 38.9 -> 13.3 us,
+// Measured against three launches of 2M-point transforms: one 128^2 map 38.9 -> 13.1 us,
 // 121 of 256^2 184 -> 106 us (38% issue active, 26 warps per SM: latency of the phases'
 // chains and barriers; 19 us for the maps' bytes at the copy peak), 16 of 768^2 527 ->
 // 190 us.  64 registers at 256 spill 340 bytes a thread and still beat 80 for scans of 121, 181
@@ -171,6 +171,18 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
         for (int sb = 0; sb < RPC / RL; sb++) {
             const int y0 = rank * RPC + sb * RL;
             const float2 *tws = fresh(tw), *dts = fresh(dtw);
+            // weights of the coefficient k = 1 (below) at the thread's first-stage points; up to 8
+            // are loaded while the rows are, more would not stay in registers
+            constexpr bool APART = M >= 32, EARLY = E <= 8;
+            auto weight = [&](int i) {
+                const int n = fftl::slot_pos<M, P::T, P::F0>(i, t);
+                return __ldg(&dts[n < M / 2 ? 4 * n + 1 : 4 * (M - 1 - n) + 3]).x;
+            };
+            float wk[EARLY ? E : 1];
+            if constexpr (APART && EARLY) {
+#pragma unroll
+                for (int i = 0; i < E; i++) wk[i] = weight(i);
+            }
             // in two halves of the lines: their rows and the ones around them by independent
             // coalesced loads, then the Laplacian into the permuted lines
 #pragma unroll 1
@@ -201,9 +213,8 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
             // over 192 maps of a specimen, that form / without the sum / with it: 2.5 / 1.8 / 1.7e-7
             // at 64, 2.2 / 2.2 / 2.0 at 128, 3.2 / 3.2 / 2.9 at 256, 4.5 / 4.9 / 4.1 at 384, 5.6 / 6.4 / 5.4
             // at 512, 9.0 / 10.0 / 7.9 at 768; over 320 maps of noise 2.2 / 2.3 / 2.0e-6 at 64, 4.0 / 4.5 /
-            // 3.9 at 128, 8.6 / 9.3 / 8.2 at 256 (16 needs none).  One map of 128^2 13.0 -> 13.3 us, 121
+            // 3.9 at 128, 8.6 / 9.3 / 8.2 at 256 (16 needs none).  One map of 128^2 13.0 -> 13.1 us, 121
             // of 256^2 103.7 -> 105.7, of 512^2 400 -> 404.
-            constexpr bool APART = M >= 32;
             Sum2 c1a, c1b;
             float2 v[E];
             if constexpr (APART) {
@@ -214,10 +225,7 @@ __global__ void __launch_bounds__(P::THREADS, RESIDENT / P::THREADS)
                 for (int i0 = 0; i0 < E; i0 += 8) {
                     float2 p[8];
 #pragma unroll
-                    for (int i = 0; i < 8; i++) {
-                        const int n = fftl::slot_pos<M, P::T, P::F0>(i0 + i, t);
-                        p[i] = cscale(v[i0 + i], __ldg(&dts[n < M / 2 ? 4 * n + 1 : 4 * (M - 1 - n) + 3]).x);
-                    }
+                    for (int i = 0; i < 8; i++) p[i] = cscale(v[i0 + i], EARLY ? wk[EARLY ? i0 + i : 0] : weight(i0 + i));
 #pragma unroll
                     for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
